@@ -204,11 +204,12 @@ void UNet::forward_features(int n, const __nv_bfloat16* input16, float* out) {
 }
 
 // Backward of one 3x3x3 layer: weight and bias gradients from (g, x); when
-// dx is given, the input gradient dx = conv(g, flipped weights).
-static void layer_backward(UNet& net, int layer, int D, int H, int W, const __nv_bfloat16* g, int g_stride,
-                           int g_offset, const __nv_bfloat16* x, int x_stride, __nv_bfloat16* dx, int dx_stride,
-                           int dx_offset, float* grad, __nv_bfloat16* wbf, __nv_bfloat16* wflip,
-                           unsigned int* error, cudaStream_t s) {
+// dx is given, the input gradient dx = conv(g, flipped weights), zero where
+// the ReLU of `mask` (the layer's input, channel stride mask_stride) was closed.
+static void layer_backward(int layer, int D, int H, int W, const __nv_bfloat16* g, int g_stride, int g_offset,
+                           const __nv_bfloat16* x, int x_stride, __nv_bfloat16* dx, int dx_stride, bool mask,
+                           float* grad, __nv_bfloat16* wbf, __nv_bfloat16* wflip, unsigned int* error,
+                           cudaStream_t s) {
     const int cin = kLayers[layer].cin, cout = kLayers[layer].cout;
     const long V = long(D) * H * W;
     WGradArgs wa{};
@@ -227,7 +228,6 @@ static void layer_backward(UNet& net, int layer, int D, int H, int W, const __nv
     launch_conv3_wgrad(wa, s);
     launch_bias_grad(V, cout, g, g_stride, g_offset, grad + bias_offset(layer), s);
     if (!dx) return;
-    launch_flip_weights(cout, cin, wbf + weight_offset(layer), wflip, s);
     ConvArgs a{};
     a.D = D;
     a.H = H;
@@ -236,15 +236,25 @@ static void layer_backward(UNet& net, int layer, int D, int H, int W, const __nv
     a.in_stride = g_stride;
     a.cin = cout;
     a.w = wflip;
+    // One input chunk: the plane-window kernel adds the taps in the order of
+    // the z-march, so the TMA-fed form may run where it applies: at 64^3 18 us
+    // against 23 with 16 output channels, but 42 against 34 with 48.
+    if (cout == 16 && cin <= 32 && conv3_runs_window(a, cin)) {
+        launch_flip_weights(cout, cin, wbf + weight_offset(layer), wflip, true, s);
+        a.w_window = wflip;
+    } else {
+        launch_flip_weights(cout, cin, wbf + weight_offset(layer), wflip, false, s);
+    }
     a.bias = nullptr;
     a.out = dx;
     a.out_stride = dx_stride;
-    a.out_offset = dx_offset;
+    a.out_offset = 0;
     a.out_fp32 = 0;
     a.relu = 0;
     a.error = error;
+    a.mask = mask ? x : nullptr;
+    a.mask_stride = x_stride;
     launch_conv3(a, cin, s);
-    (void)net;
 }
 
 void UNet::backward(int n) {
@@ -270,41 +280,32 @@ void UNet::backward(int n) {
     unsigned int* err = error_.p;
 
     // head: d(d1b) = g * w_head, masked by the ReLU of layer 9
-    launch_head_backward(V1, kHeadIn, bf(d1b_), params_.p + head_offset(), gout_.p, gA, grad + head_offset(),
+    launch_head_backward(V1, bf(d1b_), params_.p + head_offset(), gout_.p, gA, grad + head_offset(),
                          grad + head_offset() + kHeadIn, s_);
     // layer 9 (input d1a)
-    layer_backward(*this, 9, n, n, n, gA, 16, 0, bf(d1a_), 16, gB, 16, 0, grad, wb, wf, err, s_);
-    launch_relu_mask(V1, 16, bf(d1a_), 16, 0, gB, 16, 0, s_);
+    layer_backward(9, n, n, n, gA, 16, 0, bf(d1a_), 16, gB, 16, true, grad, wb, wf, err, s_);
     // layer 8 (input dec1 = [upsample(d2b) : 32 | skip1 : 16])
-    layer_backward(*this, 8, n, n, n, gB, 16, 0, bf(dec1_), 48, gdec1, 48, 0, grad, wb, wf, err, s_);
-    launch_upsample2_backward(h, h, h, 32, gdec1, 48, gl2b, s_);
-    launch_relu_mask(V2, 32, bf(d2b_), 32, 0, gl2b, 32, 0, s_);
+    layer_backward(8, n, n, n, gB, 16, 0, bf(dec1_), 48, gdec1, 48, false, grad, wb, wf, err, s_);
+    launch_upsample2_backward(h, h, h, 32, gdec1, 48, gl2b, bf(d2b_), s_);
     // layer 7 (input d2a)
-    layer_backward(*this, 7, h, h, h, gl2b, 32, 0, bf(d2a_), 32, gl2, 32, 0, grad, wb, wf, err, s_);
-    launch_relu_mask(V2, 32, bf(d2a_), 32, 0, gl2, 32, 0, s_);
+    layer_backward(7, h, h, h, gl2b, 32, 0, bf(d2a_), 32, gl2, 32, true, grad, wb, wf, err, s_);
     // layer 6 (input dec2 = [upsample(e3b) : 64 | skip2 : 32])
-    layer_backward(*this, 6, h, h, h, gl2, 32, 0, bf(dec2_), 96, gdec2, 96, 0, grad, wb, wf, err, s_);
-    launch_upsample2_backward(q, q, q, 64, gdec2, 96, gl3b, s_);
-    launch_relu_mask(V3, 64, bf(e3b_), 64, 0, gl3b, 64, 0, s_);
+    layer_backward(6, h, h, h, gl2, 32, 0, bf(dec2_), 96, gdec2, 96, false, grad, wb, wf, err, s_);
+    launch_upsample2_backward(q, q, q, 64, gdec2, 96, gl3b, bf(e3b_), s_);
     // layer 5 (input e3a)
-    layer_backward(*this, 5, q, q, q, gl3b, 64, 0, bf(e3a_), 64, gl3a, 64, 0, grad, wb, wf, err, s_);
-    launch_relu_mask(V3, 64, bf(e3a_), 64, 0, gl3a, 64, 0, s_);
+    layer_backward(5, q, q, q, gl3b, 64, 0, bf(e3a_), 64, gl3a, 64, true, grad, wb, wf, err, s_);
     // layer 4 (input e3in = pool(skip2)); its input gradient reuses gl3b as [V3][32]
-    layer_backward(*this, 4, q, q, q, gl3a, 64, 0, bf(e3in_), 32, gl3b, 32, 0, grad, wb, wf, err, s_);
-    launch_avgpool2_backward(h, h, h, 32, gl3b, gdec2, 96, 64, true, s_);
-    launch_relu_mask(V2, 32, bf(dec2_), 96, 64, gdec2, 96, 64, s_);
+    layer_backward(4, q, q, q, gl3a, 64, 0, bf(e3in_), 32, gl3b, 32, false, grad, wb, wf, err, s_);
+    launch_avgpool2_backward(h, h, h, 32, gl3b, gdec2, 96, 64, bf(dec2_), 96, 64, s_);
     // layer 3 (input e2a), output gradient gdec2[:, 64:96]
-    layer_backward(*this, 3, h, h, h, gdec2, 96, 64, bf(e2a_), 32, gl2, 32, 0, grad, wb, wf, err, s_);
-    launch_relu_mask(V2, 32, bf(e2a_), 32, 0, gl2, 32, 0, s_);
+    layer_backward(3, h, h, h, gdec2, 96, 64, bf(e2a_), 32, gl2, 32, true, grad, wb, wf, err, s_);
     // layer 2 (input e2in = pool(skip1)); its input gradient reuses gl2b as [V2][16]
-    layer_backward(*this, 2, h, h, h, gl2, 32, 0, bf(e2in_), 16, gl2b, 16, 0, grad, wb, wf, err, s_);
-    launch_avgpool2_backward(n, n, n, 16, gl2b, gdec1, 48, 32, true, s_);
-    launch_relu_mask(V1, 16, bf(dec1_), 48, 32, gdec1, 48, 32, s_);
+    layer_backward(2, h, h, h, gl2, 32, 0, bf(e2in_), 16, gl2b, 16, false, grad, wb, wf, err, s_);
+    launch_avgpool2_backward(n, n, n, 16, gl2b, gdec1, 48, 32, bf(dec1_), 48, 32, s_);
     // layer 1 (input e1a), output gradient gdec1[:, 32:48]
-    layer_backward(*this, 1, n, n, n, gdec1, 48, 32, bf(e1a_), 16, gA, 16, 0, grad, wb, wf, err, s_);
-    launch_relu_mask(V1, 16, bf(e1a_), 16, 0, gA, 16, 0, s_);
+    layer_backward(1, n, n, n, gdec1, 48, 32, bf(e1a_), 16, gA, 16, true, grad, wb, wf, err, s_);
     // layer 0 (input features): no input gradient needed
-    layer_backward(*this, 0, n, n, n, gA, 16, 0, bf(in0_), 16, nullptr, 0, 0, grad, wb, wf, err, s_);
+    layer_backward(0, n, n, n, gA, 16, 0, bf(in0_), 16, nullptr, 0, false, grad, wb, wf, err, s_);
     VB_CUDA(cudaGetLastError());
 }
 

@@ -106,6 +106,12 @@ __host__ __device__ constexpr uint32_t instr_desc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24);
 }
 
+// Bits of the instruction descriptor for MN-major operands: in the canonical
+// layout without swizzle a core matrix is then 8 K values of 8 consecutive M (N)
+// elements, one 16-byte row per K value; LBO is the distance between 8-value
+// K blocks, SBO between 8-element M (N) groups.
+constexpr uint32_t kMnMajorA = 1u << 15, kMnMajorB = 1u << 16;
+
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, bool accumulate) {
     const uint32_t acc = accumulate ? 1u : 0u;
     asm volatile(

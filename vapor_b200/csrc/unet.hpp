@@ -37,6 +37,8 @@ struct ConvArgs {
     unsigned int* error;          // bit 1: a bounded wait timed out; bit 2: in-flight MMAs could not be drained
     int wait_probe;               // test hook: > 0 makes each CTA's first completion wait poll a barrier
                                   // that nothing completes, wait_probe times, so that it runs out
+    const __nv_bfloat16* mask;    // with mask_stride channels per voxel: outputs (BF16) whose mask value is not
+    int mask_stride;              // positive are stored as 0 (the ReLU backward of an input gradient), or null
     const __nv_bfloat16* w_window;  // w packed for the plane-window kernels (launch_pack_window), or null
 };
 
@@ -64,6 +66,9 @@ void set_conv_kernel(int kind);
 // the plane-window kernels (27 cout cin values).
 void launch_pack_window(int cout, int cin, const __nv_bfloat16* w, __nv_bfloat16* packed, cudaStream_t s);
 void launch_conv3(const ConvArgs& a, int cout, cudaStream_t s);
+// Whether launch_conv3 runs the TMA-fed plane-window form for these arguments
+// when ConvArgs::w_window is given.
+bool conv3_runs_window(const ConvArgs& a, int cout);
 void launch_conv3_wgrad(const WGradArgs& a, cudaStream_t s);
 // Weight-gradient kernel: 1 (default) tcgen05 implicit GEMM, 0 the CUDA-core
 // form. Both accumulate FP32 products of the same BF16 values with atomics,
@@ -93,16 +98,18 @@ void launch_target(int n, const float* p_split, const ProjControl* ctrl, const f
 // when grad is given, its gradient with respect to p. Uses scalars[0..4].
 void launch_loss_grad(long V, const float* p, const float* t, double* partial, double* scalars, float* grad,
                       cudaStream_t s);
-void launch_head_backward(long V, int C, const __nv_bfloat16* act, const float* w, const float* g,
-                          __nv_bfloat16* dact, float* dw, float* db, cudaStream_t s);
-void launch_relu_mask(long V, int C, const __nv_bfloat16* act, int act_stride, int act_offset, __nv_bfloat16* g,
-                      int g_stride, int g_offset, cudaStream_t s);
+void launch_head_backward(long V, const __nv_bfloat16* act, const float* w, const float* g,
+                          __nv_bfloat16* dact, float* dw, float* db, cudaStream_t s);  // kHeadIn channels
 void launch_bias_grad(long V, int C, const __nv_bfloat16* g, int g_stride, int g_offset, float* db, cudaStream_t s);
-void launch_flip_weights(int cout, int cin, const __nv_bfloat16* w, __nv_bfloat16* wt, cudaStream_t s);
+// With `window` (cout = 16) the flipped weights come packed for the
+// plane-window kernels (ConvArgs::w_window of the 16 -> cin convolution).
+void launch_flip_weights(int cout, int cin, const __nv_bfloat16* w, __nv_bfloat16* wt, bool window, cudaStream_t s);
+// Both also apply the ReLU backward of `act`, the activation whose gradient they write.
 void launch_avgpool2_backward(int D, int H, int W, int C, const __nv_bfloat16* dout, __nv_bfloat16* din,
-                              int din_stride, int din_offset, bool add, cudaStream_t s);
+                              int din_stride, int din_offset, const __nv_bfloat16* act, int act_stride,
+                              int act_offset, cudaStream_t s);
 void launch_upsample2_backward(int d, int h, int w, int C, const __nv_bfloat16* dfine, int fine_stride,
-                               __nv_bfloat16* dcoarse, cudaStream_t s);
+                               __nv_bfloat16* dcoarse, const __nv_bfloat16* act, cudaStream_t s);
 void launch_adam(long count, float* w, float* m, float* v, const float* g, __nv_bfloat16* wb, float lr, int step,
                  cudaStream_t s);
 void launch_to_bf16(long count, const float* a, __nv_bfloat16* b, cudaStream_t s);

@@ -66,6 +66,26 @@ __device__ __forceinline__ void issue_taps(uint32_t d, uint64_t a_desc, const ui
             }
 }
 
+// Keeps the 8 BF16 gradients of `g` whose activation is positive (ReLU backward).
+__device__ __forceinline__ uint4 relu_mask8(uint4 g, uint4 act) {
+    const __nv_bfloat16* m = reinterpret_cast<const __nv_bfloat16*>(&act);
+    __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&g);
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+        if (!(__bfloat162float(m[c]) > 0.f)) e[c] = __float2bfloat16_rn(0.f);
+    return g;
+}
+
+// Stores 8 output channels from c0 of voxel v in BF16, masked when asked.
+__device__ __forceinline__ void store_bf16x8(const ConvArgs& a, long v, int c0, const float (&val)[8]) {
+    __align__(16) __nv_bfloat16 hv[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) hv[i] = __float2bfloat16_rn(val[i]);
+    uint4 out = *reinterpret_cast<const uint4*>(hv);
+    if (a.mask) out = relu_mask8(out, *reinterpret_cast<const uint4*>(a.mask + v * a.mask_stride + c0));
+    *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(a.out) + v * a.out_stride + a.out_offset + c0) = out;
+}
+
 // Epilogue of one tile of 128 voxels (8 x by 16 y in plane z): accumulator
 // columns [0, N) at TMEM address acc, plus bias, optional ReLU, into the
 // output (BF16 or FP32, out_stride channels per voxel from out_offset). Warp w
@@ -98,11 +118,7 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, uint32_t acc, c
                 dst[0] = make_float4(val[0], val[1], val[2], val[3]);
                 dst[1] = make_float4(val[4], val[5], val[6], val[7]);
             } else {
-                __align__(16) __nv_bfloat16 hv[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) hv[i] = __float2bfloat16_rn(val[i]);
-                *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(a.out) + o) =
-                    *reinterpret_cast<const uint4*>(hv);
+                store_bf16x8(a, v, c0, val);
             }
         }
     }
@@ -441,11 +457,7 @@ __device__ __forceinline__ void ws_epilogue(const ConvArgs& a, uint32_t acc, con
                 dst[0] = make_float4(val[0], val[1], val[2], val[3]);
                 dst[1] = make_float4(val[4], val[5], val[6], val[7]);
             } else {
-                __align__(16) __nv_bfloat16 hv[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) hv[i] = __float2bfloat16_rn(val[i]);
-                *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(a.out) + o) =
-                    *reinterpret_cast<const uint4*>(hv);
+                store_bf16x8(a, v, c0, val);
             }
         }
     }
@@ -1284,52 +1296,88 @@ __global__ void k_loss_grad(long V, const float* __restrict__ p, const float* __
         grad[v] = float(cr * (double(t[v]) - mt) + cq * (double(p[v]) - mp));
 }
 
-__global__ void k_head_backward(long V, int C, const __nv_bfloat16* __restrict__ act, const float* __restrict__ w,
-                                const float* __restrict__ g, __nv_bfloat16* __restrict__ dact,
-                                float* __restrict__ dw, float* __restrict__ db) {
-    float lw[64], lb = 0.f;
-    for (int c = 0; c < C; ++c) lw[c] = 0.f;
+// Output head backward: dact = g w masked by the ReLU of the head's input, dw
+// += sum_v g act, db += sum_v g. A voxel's kHeadIn = 16 channels are two
+// 16-byte loads and stores; the 17 sums stay in registers, are reduced in the
+// block and cost one atomic per block and value. Bound by its bytes (68 per
+// voxel). With every thread adding its own 17 values (2.6 M atomics on 17
+// addresses) a 64^3 call took 2761 us, so grid and reduction follow the
+// number of blocks, not of threads: 7.4 us.
+__global__ void __launch_bounds__(256) k_head_backward(long V, const __nv_bfloat16* __restrict__ act,
+                                                       const float* __restrict__ w, const float* __restrict__ g,
+                                                       __nv_bfloat16* __restrict__ dact, float* __restrict__ dw,
+                                                       float* __restrict__ db) {
+    constexpr int C = kHeadIn;
+    __shared__ float s_acc[8][C + 1];
+    float lw[C + 1], wr[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        lw[c] = 0.f;
+        wr[c] = w[c];
+    }
+    lw[C] = 0.f;
     for (long v = long(blockIdx.x) * blockDim.x + threadIdx.x; v < V; v += long(gridDim.x) * blockDim.x) {
         const float gv = g[v];
-        lb += gv;
-        for (int c = 0; c < C; ++c) {
-            const float a = __bfloat162float(act[v * C + c]);
-            lw[c] += gv * a;
-            dact[v * C + c] = __float2bfloat16_rn(a > 0.f ? gv * w[c] : 0.f);
+        lw[C] += gv;
+        const uint4* src = reinterpret_cast<const uint4*>(act + v * C);
+        uint4* dst = reinterpret_cast<uint4*>(dact + v * C);
+#pragma unroll
+        for (int h = 0; h < C / 8; ++h) {
+            const uint4 in = src[h];
+            const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&in);
+            __align__(16) __nv_bfloat16 o[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const float x = __bfloat162float(e[c]);
+                lw[8 * h + c] += gv * x;
+                o[c] = __float2bfloat16_rn(x > 0.f ? gv * wr[8 * h + c] : 0.f);
+            }
+            dst[h] = *reinterpret_cast<const uint4*>(o);
         }
     }
-    for (int c = 0; c < C; ++c) atomicAdd(&dw[c], lw[c]);
-    atomicAdd(db, lb);
-}
-
-// ReLU backward in place on a gradient with channel stride: g *= (act > 0).
-__global__ void k_relu_mask(long V, int C, const __nv_bfloat16* __restrict__ act, int act_stride, int act_offset,
-                            __nv_bfloat16* __restrict__ g, int g_stride, int g_offset) {
-    const long total = V * C;
-    for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
-        const int c = int(i % C);
-        const long v = i / C;
-        if (!(__bfloat162float(act[v * act_stride + act_offset + c]) > 0.f))
-            g[v * g_stride + g_offset + c] = __float2bfloat16_rn(0.f);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int c = 0; c <= C; ++c) {
+        const float t = warp_sum(lw[c]);
+        if (lane == 0) s_acc[warp][c] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x <= C) {
+        float t = 0.f;
+        for (int k = 0; k < 8; ++k) t += s_acc[k][threadIdx.x];
+        atomicAdd(threadIdx.x < C ? &dw[threadIdx.x] : db, t);
     }
 }
 
-// Bias gradient: db[co] += sum_v g[v, co].
-__global__ void k_bias_grad(long V, int C, const __nv_bfloat16* __restrict__ g, int g_stride, int g_offset,
-                            float* __restrict__ db) {
-    __shared__ float s_acc[128];
-    if (threadIdx.x < C) s_acc[threadIdx.x] = 0.f;
+// Bias gradient: db[co] += sum_v g[v, co], 8 channels (16 bytes) a thread (C =
+// 16, 32 or 64, stride and offset multiples of 8). The lanes of a warp that
+// hold the same channels reduce by shuffles, the warps through shared memory;
+// one atomic per block and channel. Reading 2 bytes a thread it took 8 us a
+// call at 64^3 x 16 channels, now 6.5.
+__global__ void __launch_bounds__(256) k_bias_grad(long V, int C, const __nv_bfloat16* __restrict__ g, int g_stride,
+                                                   int g_offset, float* __restrict__ db) {
+    __shared__ float s_acc[8][64];
+    const int groups = C / 8, group = threadIdx.x % groups;
+    const long lanes = blockDim.x / groups;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (long v = long(blockIdx.x) * lanes + threadIdx.x / groups; v < V; v += long(gridDim.x) * lanes) {
+        const uint4 in = *reinterpret_cast<const uint4*>(g + v * g_stride + g_offset + group * 8);
+        const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&in);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc[c] += __bfloat162float(e[c]);
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        for (int o = 16; o >= groups; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+        if (lane < groups) s_acc[warp][lane * 8 + c] = acc[c];
+    }
     __syncthreads();
-    const int c = threadIdx.x % C;
-    const int lanes = blockDim.x / C;
-    const int l = threadIdx.x / C;
-    float acc = 0.f;
-    if (l < lanes)
-        for (long v = long(blockIdx.x) * lanes + l; v < V; v += long(gridDim.x) * lanes)
-            acc += __bfloat162float(g[v * g_stride + g_offset + c]);
-    if (l < lanes) atomicAdd(&s_acc[c], acc);
-    __syncthreads();
-    if (threadIdx.x < C) atomicAdd(&db[threadIdx.x], s_acc[threadIdx.x]);
+    if (threadIdx.x < C) {
+        float t = 0.f;
+        for (int k = 0; k < 8; ++k) t += s_acc[k][threadIdx.x];
+        atomicAdd(&db[threadIdx.x], t);
+    }
 }
 
 // Weight gradient of a 3x3x3 convolution on CUDA cores:
@@ -1376,25 +1424,27 @@ __global__ void __launch_bounds__(256) k_conv3_wgrad(WGradArgs a) {
 // a GEMM per CTA: M = 128 rows (8 taps x 16 output channels of one chunk), N
 // = cin, K = the voxels of the CTA's range. Shared memory holds, per stage
 // of 64 voxels, A[(tap, co)][v'] = g[v' - t][co] (zero where v' - t leaves
-// the grid) and B[ci][v'] = x[v'][ci], both in the canonical K-major layout
-// without swizzle ([8-row group][8-voxel chunk][8 rows][16 B]: LBO 128 B, SBO
-// 1024 B), staged by all threads (each voxel's channels scattered down one K
-// column); one thread issues the 4 MMAs (K = 16) of a stage into the FP32
-// TMEM accumulator, two stages alternate on commit barriers. The epilogue
-// adds the accumulator to dW with FP32 atomics, as the CUDA-core form does.
+// the grid) and B[ci][v'] = x[v'][ci]. Both are stored MN-major: a voxel's 8
+// channels are one 16-byte row, 8 voxels a core matrix, so the channels-last
+// activations are copied as they are, 16 bytes a store ([8-row group][voxel]
+// [16 B]: 1024 B between row groups, 128 B between 8-voxel blocks). The
+// registers of the next stage are loaded while the MMAs of this one run. One
+// thread issues the 4 MMAs (K = 16) of a stage into the FP32 TMEM
+// accumulator, two stages alternate on commit barriers. The epilogue adds the
+// accumulator to dW with FP32 atomics, as the CUDA-core form does.
+// Bound by the latency of the staging loads (g is read once per tap from
+// L2); a K-major stage, with every channel scattered to a row of its own (2
+// bytes a store), took 165 us at 64^3 x 16 x 16 and this one 80 us.
 struct WGradTc {
     static constexpr int kK = 64;                 // voxels per stage
-    static constexpr int kA = 128 * kK * 2;       // 16 KB
-    __host__ __device__ static int b_bytes(int cin) { return cin * kK * 2; }
+    static constexpr int kGroup = kK * 16;        // 8 rows (channels) of a stage
+    static constexpr int kA = 16 * kGroup;        // 16 KB
+    __host__ __device__ static int b_bytes(int cin) { return cin / 8 * kGroup; }
     __host__ __device__ static int stage(int cin) { return kA + b_bytes(cin); }
     static int smem(int cin) { return 2 * stage(cin) + 1024; }
 };
 
-__device__ __forceinline__ uint32_t kmajor_offset(int row, int k) {
-    return uint32_t((row >> 3) * 1024 + (k >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2);
-}
-
-__global__ void __launch_bounds__(256) k_conv3_wgrad_tc(WGradArgs a, long chunk) {
+__global__ void __launch_bounds__(256, 4) k_conv3_wgrad_tc(WGradArgs a, int chunk) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bars[2];
     __shared__ uint32_t tmem_slot;
@@ -1402,9 +1452,9 @@ __global__ void __launch_bounds__(256) k_conv3_wgrad_tc(WGradArgs a, long chunk)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int group = blockIdx.y;                     // taps 8 group .. 8 group + 7
     const int cob = blockIdx.z;                       // output channels 16 cob .. + 15
-    const long V = long(a.D) * a.H * a.W;
-    const long v_begin = long(blockIdx.x) * chunk, v_end = min(V, v_begin + chunk);
-    const int cin = a.cin;
+    const int V = a.D * a.H * a.W;
+    const int v_begin = int(blockIdx.x) * chunk, v_end = min(V, v_begin + chunk);
+    const int cin = a.cin, channel_groups = cin / 8;
     const uint32_t ncols = cin <= 32 ? 32u : (cin <= 64 ? 64u : 128u);
     const uint32_t sbase = tc::smem_addr(smem);
     const uint32_t bar0 = tc::smem_addr(&bars[0]);
@@ -1418,11 +1468,41 @@ __global__ void __launch_bounds__(256) k_conv3_wgrad_tc(WGradArgs a, long chunk)
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    const uint32_t idesc = tc::instr_desc_bf16(128, cin);
+    const uint32_t idesc = tc::instr_desc_bf16(128, cin) | tc::kMnMajorA | tc::kMnMajorB;
+    // Thread (voxel k, part q): of a stage it copies A's taps q and q + 4 and
+    // B's channel groups q, q + 4 and q + 8.
+    const int k = tid & 63, q = tid >> 6;
+    uint4 ra[2][2], rb[3];
+    auto load = [&](int k0) {
+        const uint4 zero = make_uint4(0, 0, 0, 0);
+        const int v = k0 + k;
+        const bool in = v < v_end;
+        const int r = v / a.W, x = v - r * a.W, z = r / a.H, y = r - z * a.H;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int t = group * 8 + q + 4 * i;
+            const int tz = t / 9, ty = (t - 9 * tz) / 3, tx = t - 9 * tz - 3 * ty;
+            const int xs = x - (tx - 1), ys = y - (ty - 1), zs = z - (tz - 1);
+            ra[i][0] = ra[i][1] = zero;
+            if (in && t < 27 && xs >= 0 && xs < a.W && ys >= 0 && ys < a.H && zs >= 0 && zs < a.D) {
+                const uint4* src = reinterpret_cast<const uint4*>(
+                    a.g + (long(zs * a.H + ys) * a.W + xs) * a.g_stride + a.g_offset + cob * 16);
+                ra[i][0] = __ldg(src);
+                ra[i][1] = __ldg(src + 1);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const int cg = q + 4 * i;
+            rb[i] = zero;
+            if (in && cg < channel_groups) rb[i] = __ldg(reinterpret_cast<const uint4*>(a.x + long(v) * a.x_stride + cg * 8));
+        }
+    };
     int issued[2] = {0, 0};
     bool ok = true;
     int s_idx = 0;
-    for (long k0 = v_begin; k0 < v_end; k0 += WGradTc::kK, s_idx ^= 1) {
+    if (v_begin < v_end) load(v_begin);
+    for (int k0 = v_begin; k0 < v_end; k0 += WGradTc::kK, s_idx ^= 1) {
         uint8_t* st = smem + s_idx * WGradTc::stage(cin);
         const uint32_t sa = sbase + uint32_t(s_idx * WGradTc::stage(cin));
         // the MMAs that last read this stage must be done
@@ -1433,49 +1513,24 @@ __global__ void __launch_bounds__(256) k_conv3_wgrad_tc(WGradArgs a, long chunk)
                 break;
             }
         }
-        // A: (tap j, voxel k) -> 16 channels of g at v' - t
-        for (int i = tid; i < 8 * WGradTc::kK; i += blockDim.x) {
-            const int j = i / WGradTc::kK, k = i - j * WGradTc::kK;
-            const int t = group * 8 + j;
-            const long v = k0 + k;
-            uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
-            if (t < 27 && v < v_end) {
-                int x, y, z;
-                decode(v, a.H, a.W, x, y, z);
-                const int xs = x - (t % 3 - 1), ys = y - ((t / 3) % 3 - 1), zs = z - (t / 9 - 1);
-                if (xs >= 0 && xs < a.W && ys >= 0 && ys < a.H && zs >= 0 && zs < a.D) {
-                    const uint4* src = reinterpret_cast<const uint4*>(
-                        a.g + ((long(zs) * a.H + ys) * a.W + xs) * a.g_stride + a.g_offset + cob * 16);
-                    lo = src[0];
-                    hi = src[1];
-                }
-            }
-            const uint16_t* e0 = reinterpret_cast<const uint16_t*>(&lo);
-            const uint16_t* e1 = reinterpret_cast<const uint16_t*>(&hi);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                *reinterpret_cast<uint16_t*>(st + kmajor_offset(j * 16 + c, k)) = e0[c];
-                *reinterpret_cast<uint16_t*>(st + kmajor_offset(j * 16 + 8 + c, k)) = e1[c];
-            }
+        for (int i = 0; i < 2; ++i) {
+            uint8_t* row = st + (2 * (q + 4 * i)) * WGradTc::kGroup + k * 16;
+            *reinterpret_cast<uint4*>(row) = ra[i][0];
+            *reinterpret_cast<uint4*>(row + WGradTc::kGroup) = ra[i][1];
         }
-        // B: (8-channel group, voxel k) -> x at v'
-        uint8_t* sb = st + WGradTc::kA;
-        for (int i = tid; i < (cin / 8) * WGradTc::kK; i += blockDim.x) {
-            const int cg = i / WGradTc::kK, k = i - cg * WGradTc::kK;
-            const long v = k0 + k;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (v < v_end) val = *reinterpret_cast<const uint4*>(a.x + v * a.x_stride + cg * 8);
-            const uint16_t* e = reinterpret_cast<const uint16_t*>(&val);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) *reinterpret_cast<uint16_t*>(sb + kmajor_offset(cg * 8 + c, k)) = e[c];
-        }
+        for (int i = 0; i < 3; ++i)
+            if (q + 4 * i < channel_groups)
+                *reinterpret_cast<uint4*>(st + WGradTc::kA + (q + 4 * i) * WGradTc::kGroup + k * 16) = rb[i];
+        if (k0 + WGradTc::kK < v_end) load(k0 + WGradTc::kK);
         tc::fence_proxy_async();  // generic-proxy stores visible to the tensor core
         tc::tc_fence_before();
         __syncthreads();
         if (tid == 0) {
             tc::tc_fence_after();
-            const uint64_t ad = tc::smem_desc(sa, 128, 1024);
-            const uint64_t bd = tc::smem_desc(sa + WGradTc::kA, 128, 1024);
+            const uint64_t ad = tc::smem_desc(sa, 128, WGradTc::kGroup);
+            const uint64_t bd = tc::smem_desc(sa + WGradTc::kA, 128, WGradTc::kGroup);
 #pragma unroll
             for (int kk = 0; kk < WGradTc::kK / 16; ++kk)
                 tc::mma_bf16(tmem, ad + uint32_t(kk * 16), bd + uint32_t(kk * 16), idesc, k0 > v_begin || kk > 0);
@@ -1485,19 +1540,19 @@ __global__ void __launch_bounds__(256) k_conv3_wgrad_tc(WGradArgs a, long chunk)
     }
     // the last commit of each stage covers every earlier MMA
     bool drained = true;
-    for (int k = 0; k < 2; ++k)
-        if (issued[k] > 0) drained &= tc::mbar_wait(bar0 + 8u * k, uint32_t(issued[k] - 1) & 1u, kWaitLimit);
+    for (int i = 0; i < 2; ++i)
+        if (issued[i] > 0) drained &= tc::mbar_wait(bar0 + 8u * i, uint32_t(issued[i] - 1) & 1u, kWaitLimit);
     ok = __syncthreads_and(ok && drained) != 0;
     tc::tc_fence_after();
     if (ok && v_begin < v_end) {
         // rows (tap j, co) on TMEM lanes; columns ci, half of them per warp pair
-        const int q = warp & 3, hlf = warp >> 2;
-        const int row = q * 32 + lane;
+        const int quarter = warp & 3, hlf = warp >> 2;
+        const int row = quarter * 32 + lane;
         const int t = group * 8 + row / 16, co = cob * 16 + (row & 15);
         const int half = cin / 2;
         for (int c0 = hlf * half; c0 < (hlf + 1) * half; c0 += 8) {
             float val[8];
-            tc::tmem_ld8(tmem + (uint32_t(q * 32) << 16) + uint32_t(c0), val);
+            tc::tmem_ld8(tmem + (uint32_t(quarter * 32) << 16) + uint32_t(c0), val);
             if (t < 27) {
 #pragma unroll
                 for (int c = 0; c < 8; ++c) atomicAdd(&a.dw[(long(t) * a.cout + co) * cin + c0 + c], val[c]);
@@ -1512,53 +1567,73 @@ __global__ void __launch_bounds__(256) k_conv3_wgrad_tc(WGradArgs a, long chunk)
 }
 
 // Flip and transpose 3x3x3 weights for the input-gradient convolution:
-// wt[26 - tap][ci][co] = w[tap][co][ci] (BF16).
+// wt[26 - tap][ci][co] = w[tap][co][ci] (BF16), or with `window` (cout = 16:
+// one input chunk) the same values in the plane-window kernels' image
+// (k_pack_window's layout of a 16 -> cin convolution).
 __global__ void k_flip_weights(int cout, int cin, const __nv_bfloat16* __restrict__ w,
-                               __nv_bfloat16* __restrict__ wt) {
+                               __nv_bfloat16* __restrict__ wt, int window) {
     const long total = 27L * cout * cin;
     for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
         const int ci = int(i % cin);
         const long r = i / cin;
         const int co = int(r % cout);
-        const int tap = int(r / cout);
-        wt[(long(26 - tap) * cin + ci) * cout + co] = w[i];
+        const int t = 26 - int(r / cout);
+        if (!window) {
+            wt[(long(t) * cin + ci) * cout + co] = w[i];
+        } else {
+            const int row = t / 9 * cin + ci;
+            wt[long(t % 9) * 3 * cin * 16 + (row >> 3) * 128 + (co >> 3) * 64 + (row & 7) * 8 + (co & 7)] = w[i];
+        }
     }
 }
 
-// avgpool backward: d_in[fine] = d_out[coarse] / 8 (into channels with stride).
+// avgpool backward, added to the skip connection's gradient, and the ReLU of
+// the pooled activation: din[fine] = (din[fine] + dout[coarse] / 8) where act >
+// 0, else 0. 8 channels (16 bytes) a thread.
 __global__ void k_avgpool2_backward(int D, int H, int W, int C, const __nv_bfloat16* __restrict__ dout,
-                                    __nv_bfloat16* __restrict__ din, int din_stride, int din_offset, int add) {
-    const long total = long(D) * H * W * C;
-    const int h = H / 2, w = W / 2;
-    for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
-        const int c = int(i % C);
-        const long v = i / C;
-        int x, y, z;
-        decode(v, H, W, x, y, z);
-        float g = __bfloat162float(dout[((long(z / 2) * h + y / 2) * w + x / 2) * C + c]) * 0.125f;
-        __nv_bfloat16& o = din[v * din_stride + din_offset + c];
-        if (add) g += __bfloat162float(o);
-        o = __float2bfloat16_rn(g);
+                                    __nv_bfloat16* __restrict__ din, int din_stride, int din_offset,
+                                    const __nv_bfloat16* __restrict__ act, int act_stride, int act_offset) {
+    const int C8 = C / 8, h = H / 2, w = W / 2;
+    const int total = D * H * W * C8;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const int v = i / C8, c = (i - v * C8) * 8;
+        const int r = v / W, x = v - r * W, z = r / H, y = r - z * H;
+        const uint4 gv = *reinterpret_cast<const uint4*>(dout + (long(z / 2 * h + y / 2) * w + x / 2) * C + c);
+        uint4* o = reinterpret_cast<uint4*>(din + long(v) * din_stride + din_offset + c);
+        uint4 ov = *o;
+        const __nv_bfloat16* ge = reinterpret_cast<const __nv_bfloat16*>(&gv);
+        __nv_bfloat16* oe = reinterpret_cast<__nv_bfloat16*>(&ov);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            oe[k] = __float2bfloat16_rn(__bfloat162float(ge[k]) * 0.125f + __bfloat162float(oe[k]));
+        *o = relu_mask8(ov, *reinterpret_cast<const uint4*>(act + long(v) * act_stride + act_offset + c));
     }
 }
 
-// upsample backward: d_coarse[c] = sum of the 8 fine gradients of channel c.
+// upsample backward and the ReLU of the upsampled activation: d_coarse[c] =
+// sum of the 8 fine gradients of channel c where act > 0. 8 channels a thread.
 __global__ void k_upsample2_backward(int d, int h, int w, int C, const __nv_bfloat16* __restrict__ dfine,
-                                     int fine_stride, __nv_bfloat16* __restrict__ dcoarse) {
-    const long total = long(d) * h * w * C;
-    const int H = 2 * h, W = 2 * w;
-    for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
-        const int c = int(i % C);
-        const long v = i / C;
-        int x, y, z;
-        decode(v, h, w, x, y, z);
-        float s = 0.f;
+                                     int fine_stride, __nv_bfloat16* __restrict__ dcoarse,
+                                     const __nv_bfloat16* __restrict__ act) {
+    const int C8 = C / 8, H = 2 * h, W = 2 * w;
+    const int total = d * h * w * C8;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const int v = i / C8, c = (i - v * C8) * 8;
+        const int r = v / w, x = v - r * w, z = r / h, y = r - z * h;
+        float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int xx = 2 * x + (k & 1), yy = 2 * y + ((k >> 1) & 1), zz = 2 * z + (k >> 2);
-            s += __bfloat162float(dfine[((long(zz) * H + yy) * W + xx) * fine_stride + c]);
+            const uint4 fv = *reinterpret_cast<const uint4*>(dfine + (long(zz * H + yy) * W + xx) * fine_stride + c);
+            const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&fv);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s[j] += __bfloat162float(e[j]);
         }
-        dcoarse[v * C + c] = __float2bfloat16_rn(s);
+        __align__(16) __nv_bfloat16 o[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = __float2bfloat16_rn(s[j]);
+        *reinterpret_cast<uint4*>(dcoarse + long(v) * C + c) =
+            relu_mask8(*reinterpret_cast<const uint4*>(o), *reinterpret_cast<const uint4*>(act + long(v) * C + c));
     }
 }
 
@@ -1659,6 +1734,16 @@ int resident_ws(int smem) {
                                  kSmemPerSm / (smem + kPerCta)}));
 }
 
+// The TMA-fed form applies: an input aligned for its boxes and a grid at
+// least as wide as the 10 x 18 box (it also needs ConvArgs::w_window).
+template <int N>
+bool window_applies(const ConvArgs& a) {
+    if constexpr (ConvWindow<N>::kSupported)
+        return g_conv_kind.load() == 3 && ConvTma<N>::fits(a.cin, 3, 2) && a.W >= 10 && a.H >= 18 &&
+               (reinterpret_cast<uintptr_t>(a.in) & 15) == 0;
+    return false;
+}
+
 template <int N>
 void launch_conv_n(const ConvArgs& a, cudaStream_t s) {
     if (a.cin % 16 != 0 || a.in_stride % 8 != 0 || a.out_stride % 8 != 0 || a.out_offset % 8 != 0)
@@ -1668,11 +1753,7 @@ void launch_conv_n(const ConvArgs& a, cudaStream_t s) {
     const int kind = g_conv_kind.load();
     bool done = false;
     if constexpr (ConvWindow<N>::kSupported) {
-        // the TMA-fed form: packed weights, a 16-byte aligned input, and a
-        // grid at least as wide as the 10 x 18 box
-        const bool tma = kind == 3 && a.w_window != nullptr && ConvTma<N>::fits(a.cin, 3, 2) && a.W >= 10 &&
-                         a.H >= 18 && (reinterpret_cast<uintptr_t>(a.in) & 15) == 0;
-        if (tma) {
+        if (a.w_window != nullptr && window_applies<N>(a)) {
             // planes per CTA and ring depth: the pair that minimises waves x
             // (planes + 2), the input planes a CTA multiplies; resident CTAs
             // by shared memory and by TMEM columns (512 per SM); on ties the
@@ -1777,6 +1858,16 @@ void launch_pack_window(int cout, int cin, const __nv_bfloat16* w, __nv_bfloat16
     k_pack_window<<<blocks_for(27L * cout * cin / 8), 256, 0, s>>>(cout, cin, w, packed);
 }
 
+bool conv3_runs_window(const ConvArgs& a, int cout) {
+    switch (cout) {
+        case 16: return window_applies<16>(a);
+        case 32: return window_applies<32>(a);
+        case 48: return window_applies<48>(a);
+        case 64: return window_applies<64>(a);
+        default: return false;
+    }
+}
+
 void launch_conv3(const ConvArgs& a, int cout, cudaStream_t s) {
     switch (cout) {
         case 16: launch_conv_n<16>(a, s); break;
@@ -1799,15 +1890,17 @@ void launch_conv3_wgrad(const WGradArgs& a, cudaStream_t s) {
     const long V = long(a.D) * a.H * a.W;
     if (g_wgrad_kind.load() == 1 && a.cin <= 96 && a.cout % 16 == 0 && a.cin % 16 == 0 &&
         a.g_stride % 8 == 0 && a.g_offset % 8 == 0 && a.x_stride % 8 == 0) {
-        // voxel ranges: about two waves of CTAs over the tap groups and
-        // output-channel chunks, at least one stage of voxels each
+        // voxel ranges: about four resident CTAs per SM over the tap groups
+        // and output-channel chunks, the most the registers allow, so that
+        // the staging loads' latency overlaps between CTAs; at least one
+        // stage of voxels each
         const int others = 4 * (a.cout / 16);
-        const long target = std::max<long>(1, (2L * device_sm_count() + others - 1) / others);
+        const long target = std::max<long>(1, 4L * device_sm_count() / others);
         const long chunk = std::max<long>(WGradTc::kK, ((V + target - 1) / target + WGradTc::kK - 1) /
                                                            WGradTc::kK * WGradTc::kK);
         const dim3 grid(unsigned((V + chunk - 1) / chunk), 4, unsigned(a.cout / 16));
         count_launch();
-        k_conv3_wgrad_tc<<<grid, 256, WGradTc::smem(a.cin), s>>>(a, chunk);
+        k_conv3_wgrad_tc<<<grid, 256, WGradTc::smem(a.cin), s>>>(a, int(chunk));
         return;
     }
     const int chunks = int(std::max<long>(1, std::min<long>(V / 4096, 256)));
@@ -1902,39 +1995,35 @@ void launch_loss_grad(long V, const float* p, const float* t, double* partial, d
     }
 }
 
-void launch_head_backward(long V, int C, const __nv_bfloat16* act, const float* w, const float* g,
+void launch_head_backward(long V, const __nv_bfloat16* act, const float* w, const float* g,
                           __nv_bfloat16* dact, float* dw, float* db, cudaStream_t s) {
     count_launch();
-    k_head_backward<<<std::min(blocks_for(V), 592), 256, 0, s>>>(V, C, act, w, g, dact, dw, db);
-}
-
-void launch_relu_mask(long V, int C, const __nv_bfloat16* act, int act_stride, int act_offset, __nv_bfloat16* g,
-                      int g_stride, int g_offset, cudaStream_t s) {
-    count_launch();
-    k_relu_mask<<<blocks_for(V * C), 256, 0, s>>>(V, C, act, act_stride, act_offset, g, g_stride, g_offset);
+    k_head_backward<<<std::min(blocks_for(V), 148 * 4), 256, 0, s>>>(V, act, w, g, dact, dw, db);
 }
 
 void launch_bias_grad(long V, int C, const __nv_bfloat16* g, int g_stride, int g_offset, float* db, cudaStream_t s) {
     count_launch();
-    k_bias_grad<<<std::min(blocks_for(V), 1184), 256, 0, s>>>(V, C, g, g_stride, g_offset, db);
+    k_bias_grad<<<std::min(blocks_for(V * (C / 8)), 148 * 4), 256, 0, s>>>(V, C, g, g_stride, g_offset, db);
 }
 
-void launch_flip_weights(int cout, int cin, const __nv_bfloat16* w, __nv_bfloat16* wt, cudaStream_t s) {
+void launch_flip_weights(int cout, int cin, const __nv_bfloat16* w, __nv_bfloat16* wt, bool window, cudaStream_t s) {
     count_launch();
-    k_flip_weights<<<blocks_for(27L * cout * cin), 256, 0, s>>>(cout, cin, w, wt);
+    k_flip_weights<<<blocks_for(27L * cout * cin), 256, 0, s>>>(cout, cin, w, wt, window ? 1 : 0);
 }
 
 void launch_avgpool2_backward(int D, int H, int W, int C, const __nv_bfloat16* dout, __nv_bfloat16* din,
-                              int din_stride, int din_offset, bool add, cudaStream_t s) {
+                              int din_stride, int din_offset, const __nv_bfloat16* act, int act_stride,
+                              int act_offset, cudaStream_t s) {
     count_launch();
-    k_avgpool2_backward<<<blocks_for(long(D) * H * W * C), 256, 0, s>>>(D, H, W, C, dout, din, din_stride,
-                                                                         din_offset, add ? 1 : 0);
+    k_avgpool2_backward<<<blocks_for(long(D) * H * W * C / 8), 256, 0, s>>>(D, H, W, C, dout, din, din_stride,
+                                                                            din_offset, act, act_stride, act_offset);
 }
 
 void launch_upsample2_backward(int d, int h, int w, int C, const __nv_bfloat16* dfine, int fine_stride,
-                               __nv_bfloat16* dcoarse, cudaStream_t s) {
+                               __nv_bfloat16* dcoarse, const __nv_bfloat16* act, cudaStream_t s) {
     count_launch();
-    k_upsample2_backward<<<blocks_for(long(d) * h * w * C), 256, 0, s>>>(d, h, w, C, dfine, fine_stride, dcoarse);
+    k_upsample2_backward<<<blocks_for(long(d) * h * w * C / 8), 256, 0, s>>>(d, h, w, C, dfine, fine_stride, dcoarse,
+                                                                             act);
 }
 
 void launch_adam(long count, float* w, float* m, float* v, const float* g, __nv_bfloat16* wb, float lr, int step,
