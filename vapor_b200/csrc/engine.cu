@@ -146,6 +146,7 @@ vapor_phase_timings PhaseTimer::totals() {
 Workspace::Workspace(int n, float box, cudaStream_t stream)
     : n_(n), box_(box), stream_(stream), timer_(stream) {
     validate_grid(n, box);
+    configure_sor_cluster();
     const size_t faces = size_t(n) * n * (n + 1);
     const size_t slots = rb_count(n);  // red-black split storage
     b_.allocate(slots);
@@ -487,11 +488,13 @@ void Workspace::project(const float* ui, const float* vi, const float* wi, float
     const bool mixed = solver_kind == VAPOR_SOLVER_MIXED_REFINEMENT || fpcg;
     const bool graph = capturing_;
     const int interval = o.residual_check_interval;
+    // small grids run their sweeps in one cluster, up to the next decision
+    const bool cluster = !fpcg && sor_cluster_applies(n_) && sor_block_iterations(n_) == 0;
     if (mixed) ensure_mixed();
     if (fpcg) ensure_fpcg(coarse != nullptr);
     // A device-side while loop is recorded only when the solve has one; a
     // conditional handle that no node uses makes graph instantiation fail.
-    const bool loop = graph && (mixed || !o.fixed_iterations || o.max_iterations > interval);
+    const bool loop = graph && (mixed || (!cluster && (!o.fixed_iterations || o.max_iterations > interval)));
     LoopCond cond;
     cudaGraphConditionalHandle handle = 0;
     if (loop) {
@@ -596,7 +599,20 @@ void Workspace::project(const float* ui, const float* vi, const float* wi, float
             }
             t.end(VAPOR_PHASE_RESIDUAL, 6);
         };
-        if (graph) {
+        if (cluster) {
+            auto sweep_then_recentre = [&](cudaStream_t st) {
+                t.begin(VAPOR_PHASE_SOR);
+                launch_sor_cluster_mixed(a, p_.p, r32_.p, ctrl_, st);
+                t.end(VAPOR_PHASE_SOR, 1);
+                t.begin(VAPOR_PHASE_RESIDUAL);
+                recentre_group(st, LoopCond{});
+                if (graph) launch_loop_condition(ctrl_, cond, st);
+                t.end(VAPOR_PHASE_RESIDUAL, 4);
+            };
+            if (graph) add_while_loop(s, body_stream_.s, handle, sweep_then_recentre);
+            else
+                while (!wait_done()) sweep_then_recentre(s);
+        } else if (graph) {
             const int chunk = std::max(1, std::min(interval, o.max_iterations));
             add_while_loop(s, body_stream_.s, handle, [&](cudaStream_t bs) { chunk_then_check(bs, chunk); });
         } else {
@@ -613,7 +629,12 @@ void Workspace::project(const float* ui, const float* vi, const float* wi, float
         t.end(VAPOR_PHASE_GRADIENT, finish);
     } else {
         if (warm) warm->infer_into(n_, b_.p, ctrl_, p_.p, nullptr);  // x0 = network prediction
-        if (o.fixed_iterations) {
+        if (cluster) {
+            t.begin(VAPOR_PHASE_SOR);
+            if (o.fixed_iterations) launch_sor_cluster_fixed(a, p_.p, b_.p, ctrl_, s);
+            else launch_sor_cluster_tolerance(a, p_.p, b_.p, ctrl_, s);
+            t.end(VAPOR_PHASE_SOR, 1);
+        } else if (o.fixed_iterations) {
             // Intermediate residual checks cannot change a fixed-budget solve:
             // the final residual and convergence are recomputed after the
             // pressure gauge (CpuPressureSolver3D.cpp:50-56).
@@ -659,6 +680,7 @@ void Workspace::project(const float* ui, const float* vi, const float* wi, float
 
 vapor_projection_result Workspace::last_result() {
     VB_CUDA(cudaStreamSynchronize(stream_));
+    if (ctrl_host_->sticky_nonfinite & 8u) fail(VAPOR_RUNTIME_ERROR, "a pressure sweep's neighbour wait timed out");
     if (ctrl_host_->sticky_nonfinite & 1u) fail(VAPOR_NON_FINITE, "Non-finite divergence");
     if (ctrl_host_->sticky_nonfinite & 6u) fail(VAPOR_NON_FINITE, "Non-finite MAC velocity");
     return ctrl_host_->result;

@@ -18,7 +18,7 @@ struct ProjControl {
     unsigned int div_after_bits;    // max |div| after, float bits
     int rhs_max_key, rhs_min_key;   // order keys of max/min of b = -div*h^2/dt
     unsigned long long res_bits;    // max |b - Ax| of the last residual pass, double bits
-    unsigned int nonfinite;         // bit 0: divergence before, bit 1: after, bit 2: solve
+    unsigned int nonfinite;         // bit 0: divergence before, 1: after, 2: solve; 3: a sweep's wait ran out
     unsigned int reserved0;
     // derived values
     float rhs_mean_f;               // (float)(sum b / C), subtracted from b on the fly
@@ -164,6 +164,20 @@ bool sor_fuses_measure(int n);
 // the grid has no such form (then nothing ran).
 int launch_sor_color_dot(const ProjectionArgs& a, int parity, float* x, const float* b, const float* q,
                          double* partials, int partial_capacity, ProjControl* ctrl, cudaStream_t s);
+// Small grids (sor_cluster_applies): the solve's sweeps in one launch of one
+// thread-block cluster (kernels_sor_cluster.cu), with the results, iteration
+// counts and control-block state of the one-colour launches and their checks.
+// They do nothing when ctrl->done. _fixed: every sweep of a fixed budget, on b
+// - mean; _tolerance: the tolerance-driven solve on b - mean with its FP64
+// residual checks; _mixed: sweeps of the error equation up to the next
+// re-centring (ctrl->recentre = 1). A neighbour wait that runs out sets bit 3
+// of ctrl->nonfinite. configure_sor_cluster: once per device before any.
+bool sor_cluster_applies(int n);
+void configure_sor_cluster();
+void launch_sor_cluster_fixed(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl, cudaStream_t s);
+void launch_sor_cluster_tolerance(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl,
+                                  cudaStream_t s);
+void launch_sor_cluster_mixed(const ProjectionArgs& p, float* e, const float* r32, ProjControl* ctrl, cudaStream_t s);
 // Temporally blocked form of the same sweeps (kernels_sor_blocked.cu):
 // `iterations` (1 or 2) red+black iterations in one launch, starting with
 // colour `first_colour`, bit-identical to 2 * iterations one-colour launches
