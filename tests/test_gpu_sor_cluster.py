@@ -1,9 +1,10 @@
-"""The cluster-resident sweeps of small grids against the oracle, which is
-pinned to the reference's CPU SOR: bit for bit, with the same iteration counts
-and residuals, at the sizes where the split can go wrong (one plane per CTA,
-slabs of unequal height, padded and odd rows, the largest grid and the first
-beyond it), for one divisor and a divisor per diagonal, and for right-hand sides
-whose quotients leave the range of the two-product division."""
+"""The resident sweeps of small grids (one cluster) and medium grids (the whole
+device) against the oracle, which is pinned to the reference's CPU SOR: bit for
+bit, with the same iteration counts and residuals, at the sizes where a split
+can go wrong (one plane per CTA, slabs and row blocks of unequal size, padded
+and odd rows, the largest grid of each form and the first beyond it), for one
+divisor and a divisor per diagonal, and for right-hand sides whose quotients
+leave the range of the two-product division."""
 import numpy as np
 import pytest
 
@@ -13,7 +14,7 @@ from vapor_b200.abi import (SOLVER_MIXED_REFINEMENT, SOLVER_RED_BLACK_SOR, Linea
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [2, 3, 7, 16, 17, 24, 31, 33, 45, 50, 61, 64, 65]
+SIZES = [2, 3, 7, 16, 17, 24, 31, 33, 45, 49, 50, 61, 64, 65, 72, 97, 128, 129]
 
 
 def _both(n, kind, opts, floor, scale=1.0, mask=None, omega=1.7):
@@ -91,7 +92,7 @@ def test_mixed_refinement(n, masked):
             assert r.linear_solve.final_residual == pytest.approx(ro.linear_solve.final_residual, rel=1e-9)
 
 
-@pytest.mark.parametrize("n", [33, 64])
+@pytest.mark.parametrize("n", [33, 64, 80])
 def test_a_graph_step_equals_the_eager_step(n):
     """The recorded step (fixed budget, tolerance and mixed loops) gives the
     bits of the same launches issued one by one."""
@@ -108,3 +109,30 @@ def test_a_graph_step_equals_the_eager_step(n):
             out.append(sim.download() + [np.array([sim.total_iterations()], np.float32)])
             sim.close()
         _bits(*out)
+
+
+def test_scenes_of_one_batch_share_the_device():
+    """Cluster and device-wide sweeps of one batch's scenes, on the split for
+    scenes that share the device, give each scene the bits of its own steps."""
+    sizes = (64, 96, 72, 33, 96)
+
+    def make():
+        sims = []
+        for k, n in enumerate(sizes):
+            p = vb.default_params()
+            p.use_solve_options, p.solver_kind = 1, SOLVER_MIXED_REFINEMENT if k % 2 else SOLVER_RED_BLACK_SOR
+            p.solve = LinearSolveOptions.defaults(max_iterations=120, fixed_iterations=0, relative_tolerance=1e-5)
+            sims.append(vb.MacSimulation3D(n, 1.0, p))
+        return sims
+
+    alone, together = make(), make()
+    batch = vb.Batch(together)
+    for _ in range(3):
+        batch.advance(1 / 60)
+        for s in alone:
+            s.advance(1 / 60)
+    batch.synchronize()
+    for a, b in zip(alone, together):
+        assert a.total_iterations() == b.total_iterations()
+        _bits(a.download(), b.download())
+    batch.close()

@@ -147,11 +147,13 @@ Workspace::Workspace(int n, float box, cudaStream_t stream)
     : n_(n), box_(box), stream_(stream), timer_(stream) {
     validate_grid(n, box);
     configure_sor_cluster();
+    configure_sor_grid();
     const size_t faces = size_t(n) * n * (n + 1);
     const size_t slots = rb_count(n);  // red-black split storage
     b_.allocate(slots);
     p_.allocate(slots);
     if (sor_blocked_applies(n)) x_alt_.allocate(slots);  // out-of-place blocked sweeps
+    if (n >= 50) sor_words_.allocate(sor_grid_words(n));  // device-wide resident sweeps
     fwd_.allocate(faces);
     partial_capacity_ = reduction_blocks(faces);
     partials_.allocate(size_t(partial_capacity_));
@@ -488,8 +490,14 @@ void Workspace::project(const float* ui, const float* vi, const float* wi, float
     const bool mixed = solver_kind == VAPOR_SOLVER_MIXED_REFINEMENT || fpcg;
     const bool graph = capturing_;
     const int interval = o.residual_check_interval;
-    // small grids run their sweeps in one cluster, up to the next decision
-    const bool cluster = !fpcg && sor_cluster_applies(n_) && sor_block_iterations(n_) == 0;
+    // Small and medium grids run their sweeps in one launch up to the next
+    // decision: in one cluster (16 SMs) where that is as fast, since several
+    // scenes then run side by side. Per half sweep, cluster against the whole
+    // device: 1.2 / 1.7 us at 48^3; at 50^3 fixed budgets 2.1 / 1.6 and tolerance
+    // checks 2.7 / 2.1, the mixed solver 1.8 / 1.9; at 64^3 1.9 / 1.4, 2.9 / 1.9
+    // and 1.8 / 1.6.
+    const bool in_grid = sor_words_.p && (!sor_cluster_applies(n_) || (!mixed && !shared_device_));
+    const bool cluster = !fpcg && (in_grid || sor_cluster_applies(n_)) && sor_block_iterations(n_) == 0;
     if (mixed) ensure_mixed();
     if (fpcg) ensure_fpcg(coarse != nullptr);
     // A device-side while loop is recorded only when the solve has one; a
@@ -602,7 +610,8 @@ void Workspace::project(const float* ui, const float* vi, const float* wi, float
         if (cluster) {
             auto sweep_then_recentre = [&](cudaStream_t st) {
                 t.begin(VAPOR_PHASE_SOR);
-                launch_sor_cluster_mixed(a, p_.p, r32_.p, ctrl_, st);
+                if (in_grid) launch_sor_grid_mixed(a, p_.p, r32_.p, ctrl_, sor_words_.p, shared_device_, st);
+                else launch_sor_cluster_mixed(a, p_.p, r32_.p, ctrl_, st);
                 t.end(VAPOR_PHASE_SOR, 1);
                 t.begin(VAPOR_PHASE_RESIDUAL);
                 recentre_group(st, LoopCond{});
@@ -631,7 +640,9 @@ void Workspace::project(const float* ui, const float* vi, const float* wi, float
         if (warm) warm->infer_into(n_, b_.p, ctrl_, p_.p, nullptr);  // x0 = network prediction
         if (cluster) {
             t.begin(VAPOR_PHASE_SOR);
-            if (o.fixed_iterations) launch_sor_cluster_fixed(a, p_.p, b_.p, ctrl_, s);
+            if (in_grid && o.fixed_iterations) launch_sor_grid_fixed(a, p_.p, b_.p, ctrl_, sor_words_.p, shared_device_, s);
+            else if (in_grid) launch_sor_grid_tolerance(a, p_.p, b_.p, ctrl_, sor_words_.p, shared_device_, s);
+            else if (o.fixed_iterations) launch_sor_cluster_fixed(a, p_.p, b_.p, ctrl_, s);
             else launch_sor_cluster_tolerance(a, p_.p, b_.p, ctrl_, s);
             t.end(VAPOR_PHASE_SOR, 1);
         } else if (o.fixed_iterations) {
@@ -945,7 +956,7 @@ void Simulation::prepare_step(float dt) {
 }
 
 void Simulation::record_step_for_batch(float dt) {
-    ws_.set_capturing(true);
+    ws_.set_capturing(true, true);
     try {
         record_step(dt);
     } catch (...) {

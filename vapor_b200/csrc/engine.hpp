@@ -157,7 +157,11 @@ public:
     bool has_solid() const { return fluid_ > 0.0; }
     // While true, project() records CUDA-graph nodes (the solve loops become
     // conditional while nodes) instead of driving the loop from the host.
-    void set_capturing(bool on) { capturing_ = on; }
+    // `shared`: among other scenes' steps, which run at the same time.
+    void set_capturing(bool on, bool shared = false) {
+        capturing_ = on;
+        shared_device_ = shared;
+    }
 
 private:
     void project_fpcg(const ProjectionArgs& a, unet::UNet* warm, unet::UNet* coarse, LoopCond cond,
@@ -175,6 +179,7 @@ private:
     DevArray<float> cg_p_, cg_q_, cg_z_;  // FPCG direction, A p, preconditioned residual
     DevArray<float> cg_p2_;             // second direction buffer of the fused step (n % 8 == 0)
     DevArray<float> x_alt_;             // twin of the iterate for out-of-place blocked sweeps
+    DevArray<uint8_t> sor_words_;       // exchange words of the device-wide resident sweeps (medium grids)
     DevArray<float> cg_rc_;             // FPCG coarse right-hand side ((n/4)^3, natural layout)
     DevArray<float> cg_rows_;           // FPCG restriction scratch (n^2 * n/4 row sums)
     DevArray<double> cg_partials_;
@@ -195,6 +200,7 @@ private:
     Stream body_stream_;                // records conditional-loop bodies
     Stream body_stream2_;               // records conditional bodies nested in a loop
     bool capturing_ = false;
+    bool shared_device_ = false;        // recording one of several scenes that run together
     long long total_iterations_ = 0;
     unsigned int sticky_errors_ = 0u;
     friend class Simulation;

@@ -178,6 +178,18 @@ void launch_sor_cluster_fixed(const ProjectionArgs& p, float* x, const float* b,
 void launch_sor_cluster_tolerance(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl,
                                   cudaStream_t s);
 void launch_sor_cluster_mixed(const ProjectionArgs& p, float* e, const float* r32, ProjControl* ctrl, cudaStream_t s);
+// Medium grids: the same on every SM of the device (kernels_sor_grid.cu), a
+// cooperative launch after the `words` (sor_grid_words(n) bytes of the caller's,
+// 0 where it does not apply) are cleared; `compact` on the fewest SMs, for
+// scenes that share the device.
+size_t sor_grid_words(int n);
+void configure_sor_grid();
+void launch_sor_grid_fixed(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl, unsigned char* words,
+                           bool compact, cudaStream_t s);
+void launch_sor_grid_tolerance(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl,
+                               unsigned char* words, bool compact, cudaStream_t s);
+void launch_sor_grid_mixed(const ProjectionArgs& p, float* e, const float* r32, ProjControl* ctrl,
+                           unsigned char* words, bool compact, cudaStream_t s);
 // Temporally blocked form of the same sweeps (kernels_sor_blocked.cu):
 // `iterations` (1 or 2) red+black iterations in one launch, starting with
 // colour `first_colour`, bit-identical to 2 * iterations one-colour launches
