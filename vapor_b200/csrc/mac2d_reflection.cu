@@ -12,7 +12,9 @@
 //     cell's 3x3 bounds see the new values of the four cells before it
 //     ((x-1, y-1), (x, y-1), (x+1, y-1), (x-1, y)) and the old values of the
 //     rest. Cell (x, y) therefore runs at wavefront step x + 2y (every earlier
-//     neighbour has a smaller step, every later one a larger), in one block;
+//     neighbour has a smaller step, every later one a larger), in one block
+//     (kr_limit_march) that takes from a parallel pass before it everything
+//     that does not depend on new values;
 //   - the emitter, whose random stirring draws the reference's LCG stream in
 //     patch order, runs on one device thread over the patch the host lists
 //     with the C library's expf, as the reference evaluates its weights;
@@ -26,6 +28,7 @@
 
 #include "engine.hpp"
 #include "powf_quarter.cuh"
+#include "sor_resident.cuh"
 
 namespace vb {
 namespace {
@@ -82,10 +85,9 @@ __global__ void kr_trace_cell(int n, float h, float dt, float dir, const float* 
 }
 
 // The MacCormack correction and in-place limiter
-// (ReflectionMacFluidSolver2D.hpp:178-194) as a wavefront: one block, step t
-// holds the cells with x + 2 y == t.
-__global__ void kr_limit(int n, float* __restrict__ field, const float* __restrict__ fwd,
-                         const float* __restrict__ back) {
+// (ReflectionMacFluidSolver2D.hpp:178-194) as it is written there, as a
+// wavefront: one block, step t holds the cells with x + 2 y == t.
+__device__ void limit_ordered(int n, float* field, const float* __restrict__ fwd, const float* __restrict__ back) {
     const int steps = 3 * n - 2;
     for (int t = 0; t < steps; ++t) {
         const int y_lo = max(0, (t - (n - 1) + 1) / 2), y_hi = min(n - 1, t / 2);
@@ -109,6 +111,115 @@ __global__ void kr_limit(int n, float* __restrict__ field, const float* __restri
             field[i] = clampf_std(corrected, lo, hi);
         }
         __syncthreads();
+    }
+}
+
+// The same by a march of threads along the rows. The order of a cell's bounds
+// decides only which of two equal zeros a bound is, and what a NaN does; so
+// without a NaN or a -0 among the inputs (none appears on the way then: a sum is
+// -0 only of two) the bounds are plain minima and maxima, and everything that
+// does not depend on a new value - fwd in the 3x3 neighbourhood, the old field
+// from the cell itself on - is taken together by a parallel pass beforehand.
+// Otherwise that pass sets `special` and limit_ordered runs.
+//
+// Thread y holds row y and runs two cells behind thread y - 1: the new value
+// above and one to the right reaches it by shuffle, those before it are kept.
+// Between warps of 32 rows the values pass through shared memory, the later warp
+// kChunk steps further behind, so that one block barrier per kChunk steps
+// suffices. Records and results lie in the march's order, [warp][step][lane],
+// step = x + 2 lane + 1, so every access is 32 neighbouring words, a chunk ahead
+// for the loads; records of no cell stay zero (w = 0). Bound by the chain of one
+// step: a shuffle, two minima or maxima and the clamp. 3n - 2 steps with a
+// barrier and 18 loads each took 337 us at n = 128, this 71.
+constexpr int kChunk = 8;
+__host__ __device__ inline int march_steps(int n) { return (n + 64 + 2 * kChunk - 1) / (2 * kChunk) * (2 * kChunk); }
+__device__ __forceinline__ int march_index(int n, int x, int y) {
+    return ((y >> 5) * march_steps(n) + x + 2 * (y & 31) + 1) * 32 + (y & 31);
+}
+
+__global__ void kr_limit_prepare(int n, const float* __restrict__ field, const float* __restrict__ fwd,
+                                 const float* __restrict__ back, float4* __restrict__ records,
+                                 unsigned int* __restrict__ special) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n * n) return;
+    const int y = i / n, x = i - y * n;
+    const float fw = fwd[i], fd = field[i];
+    const float corrected = fw + 0.5f * (fd - back[i]);
+    float lo = fminf(fw, fd), hi = fmaxf(fw, fd);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const int a = x + k % 3 - 1, b = y + k / 3 - 1;
+        if (a < 0 || a >= n || b < 0 || b >= n) continue;
+        const float u = fwd[a + n * b];
+        lo = fminf(lo, u);
+        hi = fmaxf(hi, u);
+        if (k < 4) continue;  // the field's new value is the march's
+        const float v = field[a + n * b];
+        lo = fminf(lo, v);
+        hi = fmaxf(hi, v);
+    }
+    records[march_index(n, x, y)] = make_float4(corrected, lo, hi, 1.f);
+    auto odd = [](float v) { return __float_as_uint(v) == 0x80000000u || v != v; };
+    if (odd(fw) || odd(fd) || odd(corrected)) atomicOr(special, 1u);
+}
+
+__global__ void __launch_bounds__(512) kr_limit_march(int n, const float4* __restrict__ records,
+                                                      const unsigned int* __restrict__ special,
+                                                      float* __restrict__ out, float* field,
+                                                      const float* __restrict__ fwd, const float* __restrict__ back) {
+    extern __shared__ float s_row[];  // [warp][steps + 64]: the warp's last row, x at x + 64
+    if (*special != 0u) {
+        limit_ordered(n, field, fwd, back);
+        return;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int steps = march_steps(n), stride = steps + 64;
+    const float none = __int_as_float(0x7fffffff);  // NaN: a minimum or maximum ignores it
+    for (int i = threadIdx.x; i < warps * stride; i += blockDim.x) s_row[i] = none;
+    __syncthreads();
+    const float4* in = records + size_t(warp) * steps * 32 + lane;
+    float* to = out + size_t(warp) * steps * 32 + lane;
+    const float* above_row = s_row + (warp > 0 ? warp - 1 : 0) * stride + 64;
+    float* last_row = s_row + warp * stride + 1;
+    const bool first_row = threadIdx.x == 0;  // nothing above
+    // new values at x - 1, x, x + 1 of the row above and at x - 1 of this
+    float a0, a1 = none, a2 = none, mine = none;
+    float4 now[kChunk], next[kChunk];
+    auto load = [&](float4 (&r)[kChunk], int base) {
+        if (base < 0 || base >= steps) return;
+#pragma unroll
+        for (int q = 0; q < kChunk; ++q) r[q] = in[(base + q) * 32];
+    };
+    auto march = [&](const float4 (&r)[kChunk], int base) {
+        if (base < 0 || base >= steps) return;
+#pragma unroll
+        for (int q = 0; q < kChunk; ++q) {
+            float above = __shfl_up_sync(0xffffffffu, mine, 1);
+            const float passed = above_row[base + q];
+            if (lane == 0) above = first_row ? none : passed;
+            a0 = a1;
+            a1 = a2;
+            a2 = above;
+            const float lo = fminf(fminf(fminf(r[q].y, a0), a1), fminf(a2, mine));
+            const float hi = fmaxf(fmaxf(fmaxf(r[q].z, a0), a1), fmaxf(a2, mine));
+            const float v = fminf(fmaxf(r[q].x, lo), hi);
+            mine = r[q].w != 0.f ? v : none;
+            to[(base + q) * 32] = v;
+            if (lane == 31) last_row[base + q] = mine;
+        }
+    };
+    // warp w is at its step (global step - w (64 + kChunk))
+    const int total = steps + (warps - 1) * (64 + kChunk);
+    int base = -warp * (64 + kChunk);
+    load(now, base);
+    for (int done = 0; done < total; done += 2 * kChunk) {
+        load(next, base + kChunk);
+        march(now, base);
+        __syncthreads();
+        load(now, base + 2 * kChunk);
+        march(next, base + kChunk);
+        __syncthreads();
+        base += 2 * kChunk;
     }
 }
 
@@ -179,6 +290,119 @@ __global__ void kr_sor(int n, int parity, float omega, float h2, float dt, const
     p[i] = (1.f - omega) * p[i] + omega * (sum - div[i] * h2 / dt) / float(max(terms, 1));
 }
 
+// Every iteration of a projection's SOR in one cluster, for grids whose rows
+// fit its CTAs (n <= 352): a thread keeps 4 slots of each parity of one row in
+// registers, the row neighbours come from shared memory, and the rows at a
+// CTA's ends go to the neighbour CTA as numbered words (sor_resident.cuh). The
+// operations per cell are kr_sor's: missing neighbours add +0 to a sum that is
+// never -0, the division by 2 or 4 is a multiplication by the exact reciprocal,
+// the one by 3 the two-product form (sor_resident.cuh) or, beyond its range,
+// the division. A half sweep took 3.2 us at n = 128 with a launch of its own and
+// takes 0.64 now, the chain of a neighbour word, shared memory and a barrier.
+__device__ __forceinline__ float divide_terms(float t, int terms) {
+    if (terms == 4) return t * 0.25f;
+    if (terms == 2) return t * 0.5f;
+    if (terms != 3) return t / float(max(terms, 1));
+    const float m = fabsf(t);
+    if (m >= 0x1p-96f && m <= 0x1p127f) return __fmaf_rn(t, 0x1.555556p-2f, __fmul_rn(t, -0x1.555556p-27f));
+    return t / 3.f;
+}
+
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) kr_sor_cluster(int n, int iterations, float omega, float h2, float dt,
+                                                       const float* __restrict__ div, float* __restrict__ p,
+                                                       unsigned int* __restrict__ error) {
+    using namespace resident;
+    extern __shared__ __align__(16) float s_p[];  // [parity][rows + 2][row], then the halo words
+    int rank, ctas;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;\n" : "=r"(ctas));
+    const int hw = (n + 1) / 2, G = (hw + 3) / 4, row = 4 * G + 4;
+    const int base = n / ctas, rem = n - base * ctas, rows = base + (rank < rem ? 1 : 0);
+    const int y0 = rank * base + min(rank, rem), max_rows = base + (rem > 0 ? 1 : 0);
+    const int parity_stride = (max_rows + 2) * row;
+    const int tid = threadIdx.x, yl = tid / G, g = tid - yl * G, i0 = 4 * g, y = y0 + yl;
+    const bool active = yl < rows;
+    const int at = (yl + 1) * row + i0;
+    const bool link_lo = active && yl == 0 && rank > 0, link_hi = active && yl == rows - 1 && rank + 1 < ctas;
+    // halo words [side][parity][half][group][16 B]
+    const uint32_t second = uint32_t(G) * 16u;
+    const uint32_t words = smem_u32(s_p) + 8u * uint32_t(parity_stride) + uint32_t(g) * 16u;
+    const uint32_t to_lo = rank > 0 ? map_to(words + 4u * second, rank - 1) : 0u;
+    const uint32_t to_hi = rank + 1 < ctas ? map_to(words, rank + 1) : 0u;
+    const int total = 2 * parity_stride + 32 * G;
+    for (int i = tid; i < total; i += blockDim.x) s_p[i] = 0.f;
+    __syncthreads();
+    float X[2][4], D[2][4];
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int x = 2 * (i0 + j) + ((y + c) & 1);
+            X[c][j] = D[c][j] = 0.f;
+            if (active && i0 + j < hw && x < n) {
+                X[c][j] = p[x + n * y];
+                D[c][j] = div[x + n * y] * h2 / dt;
+                s_p[c * parity_stride + at + j] = X[c][j];
+            }
+        }
+    cluster_barrier();
+    bool dead = false;
+    if (link_lo) send4(to_lo + 2u * second, second, X[1], 1u);
+    if (link_hi) send4(to_hi + 2u * second, second, X[1], 1u);
+    const int yterms = int(y > 0) + int(y + 1 < n);
+    const float keep = 1.f - omega;
+    uint32_t t = 0;
+    auto half_sweep = [&](auto parity) {
+        constexpr int c = decltype(parity)::value;
+        if (active) {
+            float* const so = s_p + (1 - c) * parity_stride + at;
+            if (!dead) {
+                const uint32_t from = words + uint32_t(1 - c) * 2u * second;
+                if (link_lo) dead = !receive4(from, second, so - row, t + 1u);
+                if (link_hi) dead = !receive4(from + 4u * second, second, so + row, t + 1u) || dead;
+            }
+            const int s = (y + c) & 1;
+            float up[4], down[4];
+            ld4(so - row, up);
+            ld4(so + row, down);
+            const float edge = s ? so[4] : so[-1];
+            const float* o = X[1 - c];
+            const float e[5] = {s ? o[0] : edge, s ? o[1] : o[0], s ? o[2] : o[1], s ? o[3] : o[2], s ? edge : o[3]};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int x = 2 * (i0 + j) + s;
+                float sum = 0.f;
+                sum += e[j];
+                sum += e[j + 1];
+                sum += up[j];
+                sum += down[j];
+                const int terms = yterms + int(x > 0) + int(x + 1 < n);
+                const float v = keep * X[c][j] + divide_terms(omega * (sum - D[c][j]), terms);
+                if (i0 + j < hw && x < n) X[c][j] = v;
+            }
+            *reinterpret_cast<float4*>(s_p + c * parity_stride + at) = make_float4(X[c][0], X[c][1], X[c][2], X[c][3]);
+            if (link_lo) send4(to_lo + uint32_t(c) * 2u * second, second, X[c], t + 2u);
+            if (link_hi) send4(to_hi + uint32_t(c) * 2u * second, second, X[c], t + 2u);
+        }
+        __syncthreads();
+        ++t;
+    };
+    for (int it = 0; it < iterations; ++it) {
+        half_sweep(std::integral_constant<int, 0>{});
+        half_sweep(std::integral_constant<int, 1>{});
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int x = 2 * (i0 + j) + ((y + c) & 1);
+            if (active && i0 + j < hw && x < n) p[x + n * y] = X[c][j];
+        }
+    if (dead) *error = 1u;
+    cluster_barrier();  // no CTA is written to after it exits
+}
+
 __global__ void kr_gradient(int n, float dt, float h_inv, const float* __restrict__ p, float* __restrict__ vx,
                             float* __restrict__ vy) {
     const long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -238,9 +462,14 @@ __global__ void kr_emit(int count, const int2* __restrict__ cells, const float* 
     *state = r;
 }
 
-__global__ void kr_scale(long count, float factor, float* __restrict__ a) {
-    const long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < count) a[i] *= factor;
+// smoke = factor * value; with `marched` the values of the limiter's march, in
+// its order, unless it was special.
+__global__ void kr_scale(int n, float factor, const float* values, const float* __restrict__ marched,
+                         const unsigned int* __restrict__ special, float* smoke) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n * n) return;
+    const int y = i / n, x = i - y * n;
+    smoke[i] = (marched && *special == 0u ? marched[march_index(n, x, y)] : values[i]) * factor;
 }
 __global__ void kr_copy(long count, const float* __restrict__ a, float* __restrict__ b) {
     const long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -281,6 +510,22 @@ __global__ void kr_diagnostics(int n, float h, const float* __restrict__ vx, con
 
 // ---- host side ----
 
+// Shared-memory and cluster limits of the kernels, once per device.
+void configure_kernels() {
+    static std::mutex mutex;
+    static std::set<int> devices;
+    int device = 0;
+    VB_CUDA(cudaGetDevice(&device));
+    std::lock_guard<std::mutex> lock(mutex);
+    if (!devices.insert(device).second) return;
+    VB_CUDA(cudaFuncSetAttribute(kr_limit_march, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+    for (const void* kernel :
+         {reinterpret_cast<const void*>(kr_sor_cluster<512>), reinterpret_cast<const void*>(kr_sor_cluster<1024>)}) {
+        VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
+        VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    }
+}
+
 class Mac2DReflection {
 public:
     Mac2DReflection(int n, const vapor_mac2d_refl_params& p) : n_(n), p_(p) {
@@ -289,8 +534,14 @@ public:
         for (DevArray<float>* a : {&smoke_, &fwd_, &back_, &pressure_, &div_}) a->allocate(cells);
         for (DevArray<float>* a : {&vx_, &vy_, &vxt_, &vyt_, &vxm_, &vym_, &vxh_, &vyh_}) a->allocate(faces);
         state_.allocate(1);
+        special_.allocate(1);
+        limit_.allocate(size_t(5) * ((n + 31) / 32) * march_steps(n) * 32);
+        limit_.zero(st_.s);  // records of no cell stay zero
         energy_.allocate(1);
         maxima_.allocate(2);
+        configure_kernels();
+        error_.allocate(1);
+        error_.zero(st_.s);
         reset();
     }
     ~Mac2DReflection() { cudaStreamSynchronize(st_.s); }
@@ -324,7 +575,13 @@ public:
             fail(VAPOR_INVALID_ARGUMENT, "Invalid 2D reflection step or parameters");
         walls(vx_.p, vy_.p);
         step(dt, p.buoyancy, std::exp(-p.smoke_decay / 60.f), p.source_strength, p.project_iterations);
+        uint32_t error = 0;
+        VB_CUDA(cudaMemcpyAsync(&error, error_.p, sizeof error, cudaMemcpyDeviceToHost, st_.s));
         VB_CUDA(cudaStreamSynchronize(st_.s));
+        if (error) {
+            error_.zero(st_.s);
+            fail(VAPOR_RUNTIME_ERROR, "a pressure sweep's neighbour wait timed out");
+        }
     }
 
     void upload(const float* s, const float* u, const float* v) {
@@ -362,15 +619,22 @@ private:
     long faces() const { return long(n_) * (n_ + 1); }
     void walls(float* u, float* v) { kr_walls<<<blocks_r(n_), kT, 0, st_.s>>>(n_, u, v); }
 
-    // advectScalar(smoke, dt) through the current velocity.
-    void advect_smoke(float dt) {
+    // advectScalar(smoke, dt) through the current velocity, then smoke *= decay.
+    void advect_smoke(float dt, float decay) {
         kr_trace_cell<<<blocks_r(cells()), kT, 0, st_.s>>>(n_, h(), dt, -1.f, vx_.p, vy_.p, smoke_.p, fwd_.p);
         if (!p_.mac_cormack_smoke) {
-            kr_copy<<<blocks_r(cells()), kT, 0, st_.s>>>(cells(), fwd_.p, smoke_.p);
+            kr_scale<<<blocks_r(cells()), kT, 0, st_.s>>>(n_, decay, fwd_.p, nullptr, nullptr, smoke_.p);
             return;
         }
+        special_.zero(st_.s);
         kr_trace_cell<<<blocks_r(cells()), kT, 0, st_.s>>>(n_, h(), dt, 1.f, vx_.p, vy_.p, fwd_.p, back_.p);
-        kr_limit<<<1, 512, 0, st_.s>>>(n_, smoke_.p, fwd_.p, back_.p);
+        const int warps = (n_ + 31) / 32, steps = march_steps(n_);
+        float4* const records = reinterpret_cast<float4*>(limit_.p);
+        float* const marched = limit_.p + size_t(4) * warps * steps * 32;
+        kr_limit_prepare<<<blocks_r(cells()), kT, 0, st_.s>>>(n_, smoke_.p, fwd_.p, back_.p, records, special_.p);
+        kr_limit_march<<<1, warps * 32, size_t(warps) * (steps + 64) * sizeof(float), st_.s>>>(
+            n_, records, special_.p, marched, smoke_.p, fwd_.p, back_.p);
+        kr_scale<<<blocks_r(cells()), kT, 0, st_.s>>>(n_, decay, smoke_.p, marched, special_.p, smoke_.p);
     }
 
     // emit(strength, dt): the patch of cells and weights, listed in the
@@ -412,16 +676,41 @@ private:
                                     vx_.p, vy_.p);
     }
 
+    // The iterations of one projection: in one cluster while its CTAs hold the
+    // rows (up to 16 CTAs of 1024 threads, 4 slots of each parity per thread),
+    // 2 to 8 rows each below n = 128; beyond, one launch per parity.
+    void sor(float dt, float h2, int iterations) {
+        const int n = n_, G = ((n + 1) / 2 + 3) / 4;
+        const int ctas = std::min(16, n / 2), rows = (n + ctas - 1) / ctas;
+        if (rows * G > 1024) {
+            const long per_parity = long((n + 1) / 2) * n;
+            for (int it = 0; it < iterations; ++it)
+                for (int parity = 0; parity < 2; ++parity)
+                    kr_sor<<<blocks_r(per_parity), kT, 0, st_.s>>>(n, parity, p_.sor_omega, h2, dt, div_.p, pressure_.p);
+            return;
+        }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(unsigned(ctas));
+        cfg.blockDim = dim3(unsigned((rows * G + 31) / 32 * 32));
+        cfg.dynamicSmemBytes = size_t(2 * (rows + 2) * (4 * G + 4) + 32 * G) * sizeof(float);
+        cfg.stream = st_.s;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = unsigned(ctas);
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        VB_CUDA(cudaLaunchKernelEx(&cfg, rows * G <= 512 ? kr_sor_cluster<512> : kr_sor_cluster<1024>, n, iterations,
+                                   p_.sor_omega, h2, dt, static_cast<const float*>(div_.p), pressure_.p, error_.p));
+    }
+
     // project(dt, iterations) (:235-285).
     void project(float dt, int iterations) {
         const float h_inv = 1.0f / h(), h2 = h() * h();
         walls(vx_.p, vy_.p);
         kr_divergence<<<blocks_r(cells()), kT, 0, st_.s>>>(n_, h_inv, vx_.p, vy_.p, div_.p);
         pressure_.zero(st_.s);
-        const long per_parity = long((n_ + 1) / 2) * n_;
-        for (int it = 0; it < iterations; ++it)
-            for (int parity = 0; parity < 2; ++parity)
-                kr_sor<<<blocks_r(per_parity), kT, 0, st_.s>>>(n_, parity, p_.sor_omega, h2, dt, div_.p, pressure_.p);
+        sor(dt, h2, iterations);
         kr_gradient<<<blocks_r(cells()), kT, 0, st_.s>>>(n_, dt, h_inv, pressure_.p, vx_.p, vy_.p);
         walls(vx_.p, vy_.p);
     }
@@ -432,8 +721,7 @@ private:
         const int half_iters = std::max(1, iterations / 2);
         const float half_decay = std::pow(dissipation, half * 60.0f);
         // stage 1: smoke half step through u0
-        advect_smoke(half);
-        kr_scale<<<blocks_r(cells()), kT, 0, st_.s>>>(cells(), half_decay, smoke_.p);
+        advect_smoke(half, half_decay);
         // stage 2: both components advected from u0, forces, projection
         kr_advect_vx<<<blocks_r(faces()), kT, 0, st_.s>>>(n_, h(), half, vx_.p, vy_.p, vx_.p, vxt_.p);
         kr_advect_vy<<<blocks_r(faces()), kT, 0, st_.s>>>(n_, h(), half, vx_.p, vy_.p, vy_.p, vyt_.p);
@@ -449,8 +737,7 @@ private:
         kr_hat<<<blocks_r(faces()), kT, 0, st_.s>>>(faces(), vym_.p, vyt_.p, vyh_.p);
         // stage 4: smoke through the midpoint, reflected velocity traced
         // through it, final projection
-        advect_smoke(half);
-        kr_scale<<<blocks_r(cells()), kT, 0, st_.s>>>(cells(), half_decay, smoke_.p);
+        advect_smoke(half, half_decay);
         kr_advect_vx<<<blocks_r(faces()), kT, 0, st_.s>>>(n_, h(), half, vxm_.p, vym_.p, vxh_.p, vx_.p);
         kr_advect_vy<<<blocks_r(faces()), kT, 0, st_.s>>>(n_, h(), half, vxm_.p, vym_.p, vyh_.p, vy_.p);
         project(half, half_iters);
@@ -460,7 +747,9 @@ private:
     vapor_mac2d_refl_params p_;
     Stream st_;
     DevArray<float> smoke_, fwd_, back_, pressure_, div_, vx_, vy_, vxt_, vyt_, vxm_, vym_, vxh_, vyh_;
-    DevArray<uint32_t> state_;
+    DevArray<uint32_t> state_, special_;
+    DevArray<uint32_t> error_;  // set by a sweep whose neighbour wait ran out
+    DevArray<float> limit_;  // the limiter's records and results in the march's order
     DevArray<double> energy_;
     DevArray<float> maxima_;
     DevArray<uint32_t> patch_cells_;

@@ -368,7 +368,8 @@ __global__ void __launch_bounds__(max_threads(PZ), 1) k_sor_resident(Args a) {
         constexpr bool MEASURE = decltype(measure)::value;
         // what follows from these is worked out anew each half sweep: kept
         // across them it would not fit the registers
-        asm volatile("" : "+r"(flags), "+f"(dyz), "+r"(last), "+r"(row0), "+r"(table_at));
+        asm volatile("" : "+r"(flags), "+f"(dyz), "+r"(last));
+        if (GRID || MODE == kTolerance) asm volatile("" : "+r"(row0), "+r"(table_at));
         if (GRID) fetch(1 - c, t + 1u);
         const float* __restrict__ so = s_x + (1 - c) * colour_stride + row0;
         float* __restrict__ sc = s_x + c * colour_stride + row0;
