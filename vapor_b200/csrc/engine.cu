@@ -148,11 +148,12 @@ Workspace::Workspace(int n, float box, cudaStream_t stream)
     validate_grid(n, box);
     configure_sor_cluster();
     configure_sor_grid();
+    configure_sor_wave();
     const size_t faces = size_t(n) * n * (n + 1);
     const size_t slots = rb_count(n);  // red-black split storage
     b_.allocate(slots);
     p_.allocate(slots);
-    if (sor_blocked_applies(n)) x_alt_.allocate(slots);  // out-of-place blocked sweeps
+    if (sor_blocked_applies(n)) x_alt_.allocate(slots);  // out-of-place sweeps
     if (n >= 50) sor_words_.allocate(sor_grid_words(n));  // device-wide resident sweeps
     fwd_.allocate(faces);
     partial_capacity_ = reduction_blocks(faces);
@@ -376,41 +377,48 @@ void Workspace::project_fpcg(const ProjectionArgs& a, unet::UNet* warm, unet::UN
     launch_refine_residual(a, b_.p, e, r, ctrl_, s);
     launch_check(ctrl_, 0, false, true, cond, s);
     t.end(VAPOR_PHASE_RESIDUAL, 2);
-    // The preconditioner, z = M r, with one-colour sweeps (the temporally
-    // blocked sweep measured slower at these sizes). With `dot`, the last
-    // sweep also writes the partials of z.r and z.q for beta; returns their
-    // block count, or 0 when they were not written.
+    // The preconditioner, z = M r: its smoothing in two-iteration passes where
+    // they apply (the first one leaves z in the twin of the iterate, the second
+    // ends in z), else in one-colour sweeps. With `dot`, the last sweep also
+    // writes the partials of z.r and z.q for beta; returns their block count, or
+    // 0 when they were not written.
+    const bool wave = sweeps == 2 && x_alt_.p && smooth_wave_applies(n_, mask != nullptr);
+    float* const zpre = wave ? x_alt_.p : cg_z_.p;
     auto precondition = [&](cudaStream_t st, bool dot) {
         t.begin(VAPOR_PHASE_SOR);
         // the first colour sweep starts from z = 0 (and clears the other colour)
         const bool fused_start = sor_fuses_measure(n_);
-        if (!fused_start) VB_CUDA(cudaMemsetAsync(cg_z_.p, 0, cg_z_.bytes(), st));
-        for (int j = 0; j < sweeps; ++j) {
+        if (wave) launch_smooth_wave_from_zero(smooth, zpre, r, ctrl_, st);
+        else if (!fused_start) VB_CUDA(cudaMemsetAsync(cg_z_.p, 0, cg_z_.bytes(), st));
+        for (int j = 0; j < sweeps && !wave; ++j) {
             launch_sor_color(smooth, 0, cg_z_.p, r, ctrl_, false, 0, false, st, false, false, fused_start && j == 0);
             launch_sor_color(smooth, 1, cg_z_.p, r, ctrl_, false, 0, false, st, false);
         }
-        t.end(VAPOR_PHASE_SOR, 2 * sweeps);
+        t.end(VAPOR_PHASE_SOR, wave ? 1 : 2 * sweeps);
         if (coarse) {
             t.begin(VAPOR_PHASE_COARSE);
-            launch_restrict_residual(n_, r, cg_z_.p, cg_rows_.p, cg_rc_.p, st, mask);
+            launch_restrict_residual(n_, r, zpre, cg_rows_.p, cg_rc_.p, st, mask);
             if (coarse_log_)
                 launch_log_coarse(cg_rc_.p, cg_rc_.n, coarse_log_, coarse_log_capacity_, coarse_log_counter_, st);
             coarse->set_stream(st);
             const float* zc = coarse->precondition(n_ / 4, cg_rc_.p);
             coarse->set_stream(s);
-            launch_coarse_correction(n_, cg_z_.p, zc, cg_rc_.p, cg_partials_.p, cg_, st, mask);
+            launch_coarse_correction(n_, zpre, zc, cg_rc_.p, cg_partials_.p, cg_, st, mask);
             t.end(VAPOR_PHASE_COARSE, 0);
         }
         t.begin(VAPOR_PHASE_SOR);
         int dot_blocks = 0;
-        for (int j = 0; j < sweeps; ++j) {
+        if (wave)
+            dot_blocks = launch_smooth_wave_back(smooth, zpre, cg_z_.p, r, dot ? cg_q_.p : nullptr, cg_partials_.p,
+                                                 int(cg_partials_.n), ctrl_, st);
+        for (int j = 0; j < sweeps && !wave; ++j) {
             launch_sor_color(smooth, 1, cg_z_.p, r, ctrl_, false, 0, false, st, false);
             if (dot && j + 1 == sweeps)
                 dot_blocks = launch_sor_color_dot(smooth, 0, cg_z_.p, r, cg_q_.p, cg_partials_.p,
                                                   int(cg_partials_.n), ctrl_, st);
             if (dot_blocks == 0) launch_sor_color(smooth, 0, cg_z_.p, r, ctrl_, false, 0, false, st, false);
         }
-        t.end(VAPOR_PHASE_SOR, 2 * sweeps);
+        t.end(VAPOR_PHASE_SOR, wave ? 1 : 2 * sweeps);
         return dot_blocks;
     };
     // n % 8 == 0 and no obstacles: the direction update, A p and the
@@ -546,12 +554,20 @@ void Workspace::project(const float* ui, const float* vi, const float* wi, float
                 ++launches;
             }
         } else {
-            for (int j = 0; j < k; ++j) {
+            // passes of two iterations where they apply, in pairs (out of place
+            // and back), the rest by colour
+            const int waved = mixed && per == 0 && !subtract_mean && x_alt_.p && sor_wave_applies(n_, a.diag != nullptr)
+                                  ? k / 4 * 4 : 0;
+            for (int j = 0; j < waved; j += 4) {
+                launch_sor_wave(a, x, x_alt_.p, rhs, ctrl_, first_index + j, false, st);
+                launch_sor_wave(a, x_alt_.p, x, rhs, ctrl_, first_index + j + 2, measure && j + 4 == k, st);
+            }
+            for (int j = waved; j < k; ++j) {
                 launch_sor_color(a, 0, x, rhs, ctrl_, true, first_index + j, subtract_mean, st, !mixed);
                 launch_sor_color(a, 1, x, rhs, ctrl_, true, first_index + j, subtract_mean, st, !mixed,
                                  measure && j + 1 == k);
             }
-            launches = 2LL * k;
+            launches = 2LL * k - waved / 2 * 3;
         }
         t.end(VAPOR_PHASE_SOR, launches);
     };

@@ -211,6 +211,21 @@ void set_sor_blocked_chunks(int n, int chunks);
 // colour); sor_block_iterations(n) is 0 where the blocked form does not apply.
 void set_sor_block_iterations(int iterations);
 int sor_block_iterations(int n);
+// Large unmasked grids: two red+black iterations of the divide-free relaxation
+// in one pass (kernels_sor_wave.cu), the same bits as four one-colour launches.
+// Out of place. launch_sor_wave is guarded like launch_sor_color (sweep indices
+// sweep_index and sweep_index + 1; copies when none is left) and with `measure`
+// records the residual of its last half sweep. The smoothing forms are the FPCG
+// preconditioner's: colours 0 1 0 1 from z = 0, and 1 0 1 0 with the partials of
+// z.r and z.q when `q` is given (returns their block count, 0 when not written).
+bool sor_wave_applies(int n, bool masked);
+bool smooth_wave_applies(int n, bool masked);
+void configure_sor_wave();
+void launch_sor_wave(const ProjectionArgs& p, const float* xin, float* xout, const float* b, ProjControl* ctrl,
+                     int sweep_index, bool measure, cudaStream_t s);
+void launch_smooth_wave_from_zero(const ProjectionArgs& p, float* z, const float* r, ProjControl* ctrl, cudaStream_t s);
+int launch_smooth_wave_back(const ProjectionArgs& p, const float* zin, float* zout, const float* r, const float* q,
+                            double* partials, int partial_capacity, ProjControl* ctrl, cudaStream_t s);
 // Autotuner hook: planes per thread of the z-marching colour sweep for grid
 // size n (planes <= 0 restores the automatic choice).
 void set_sor_planes(int n, int planes);
