@@ -191,9 +191,10 @@ void Workspace::reset_buffers() {
 void Workspace::clear_errors() { VB_CUDA(cudaMemsetAsync(&ctrl_->sticky_nonfinite, 0, sizeof(unsigned int), stream_)); }
 
 void Workspace::advect(int loc, float dt, float cfl, bool maccormack, const float* src, const float* u,
-                       const float* v, const float* w, float* out, float post_scale) {
+                       const float* v, const float* w, float* out, float post_scale, float* const* vel_cache) {
     timer_.begin(VAPOR_PHASE_ADVECT);
-    launch_advect(grid(), loc, dt, cfl, maccormack, src, u, v, w, fwd_.p, out, post_scale, stream_);
+    launch_advect(grid(), loc, dt, cfl, maccormack, src, u, v, w, fwd_.p, out, post_scale, vel_cache,
+                  stream_);
     timer_.end(VAPOR_PHASE_ADVECT, maccormack ? 2 : 1);
     VB_CUDA(cudaGetLastError());
 }
@@ -1377,7 +1378,9 @@ void Stage::advect(int loc, float dt, float cfl, int method, const float* src, c
         VB_CUDA(cudaMemcpyAsync(src_.p, src, count * sizeof(float), cudaMemcpyDeviceToDevice, s));
         dsrc = src_.p;
     }
-    ws_.advect(loc, dt, cfl, method == VAPOR_MACCORMACK, dsrc, dflow[0], dflow[1], dflow[2], dout, 1.f);
+    // the projection's outputs are free here: the traced velocities
+    float* const traced[3] = {out_[0].p, out_[1].p, out_[2].p};
+    ws_.advect(loc, dt, cfl, method == VAPOR_MACCORMACK, dsrc, dflow[0], dflow[1], dflow[2], dout, 1.f, traced);
     if (!device_pointers) VB_CUDA(cudaMemcpyAsync(out, dst_.p, count * sizeof(float), cudaMemcpyDeviceToHost, s));
     VB_CUDA(cudaStreamSynchronize(s));
 }

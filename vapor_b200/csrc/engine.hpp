@@ -126,7 +126,7 @@ public:
     }
     float* rhs() { return b_.p; }
     void advect(int loc, float dt, float cfl, bool maccormack, const float* src, const float* u, const float* v,
-                const float* w, float* out, float post_scale);
+                const float* w, float* out, float post_scale, float* const* vel_cache);
     // The three velocity components in one forward and one MacCormack launch
     // (their forward passes kept in a 3-face-array scratch).
     void advect_velocity(float dt, float cfl, bool maccormack, const float* const src[3], const float* u,

@@ -101,7 +101,7 @@ void launch_walls(const Grid& g, float* u, float* v, float* w, cudaStream_t s);
 // (the smoke dissipation factor; 1 for velocity).
 void launch_advect(const Grid& g, int loc, float dt, float cfl_limit, bool maccormack, const float* src,
                    const float* u, const float* v, const float* w, float* fwd, float* out, float post_scale,
-                   cudaStream_t s);
+                   float* const* vel_cache, cudaStream_t s);
 // The three velocity components src[c] (faces of axis c) through the flow
 // (u, v, w) into out[c], in one forward launch (into fwd[c]) and one
 // MacCormack launch; same results as three launch_advect calls. With

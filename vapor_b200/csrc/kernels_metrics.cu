@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kThreads) k_metrics(Grid g, float fps, float c
         // cell centre (x + .5) / n of the unit box, scaled to the box
         const float px = (float(x) + .5f) / float(n) * box, py = (float(y) + .5f) / float(n) * box,
                     pz = (float(z) + .5f) / float(n) * box;
-        const Vel vel = velocity_at(u, v, w, n, g.h, px, py, pz);
+        const Vel vel = velocity_at(u, v, w, n, cell_size<false>(g.h), px, py, pz);
         const float cfl = sqrtf(vel.x * vel.x + vel.y * vel.y + vel.z * vel.z) * float(n) / (box * fps);
         cmax = fmaxf(cmax, cfl);
         if (cfl > cfl_limit) ++cfl_fb;

@@ -46,10 +46,35 @@ __device__ __forceinline__ float maxf_ref(float a, float b) { return a < b ? b :
 // Division by the cell size as the reference writes it, coord / h, or, when h
 // is a power of two, coord * (1 / h): 1 / h is then exact, so both forms round
 // the same real quotient to the same float (also for subnormal results) and
-// the multiplication saves the IEEE division's instruction sequence.
+// the multiplication saves the IEEE division's instruction sequence. For other
+// cell sizes: with zh the rounded reciprocal and zl its rounding error,
+// coord zh + coord zl is within one unit of the quotient's last place, from
+// where one correction by the exact remainder gives the rounded quotient
+// (P. Markstein, Computation of elementary functions on the IBM RISC
+// System/6000 processor, 1990, theorem on the last step of a division), four
+// operations in the place of some ten. Where a remainder could leave the normal
+// range (and for infinities and NaN), the division itself.
+struct CellSize {
+    float h, zh, zl, most;  // most: 2^60, or 0 where h itself is out of the range
+};
 template <bool POW2>
-__device__ __forceinline__ float div_h(float coord, float h, float ih) {
-    return POW2 ? coord * ih : coord / h;
+__device__ __forceinline__ CellSize cell_size(float h) {
+    CellSize c;
+    c.h = h;
+    c.zh = 1.f / h;
+    c.zl = POW2 ? 0.f : __fmaf_rn(-c.zh, h, 1.f) * c.zh;
+    c.most = h > 0x1p-30f && h < 0x1p30f ? 0x1p60f : 0.f;
+    return c;
+}
+template <bool POW2>
+__device__ __forceinline__ float div_h(float coord, const CellSize& c) {
+    if (POW2) return coord * c.zh;
+    const float size = fabsf(coord);
+    if (size < c.most && (size > 0x1p-60f || __float_as_uint(coord) == 0u)) {
+        const float q = __fmaf_rn(coord, c.zh, coord * c.zl);
+        return __fmaf_rn(__fmaf_rn(-q, c.h, coord), c.zh, q);
+    }
+    return coord / c.h;
 }
 
 // One axis of the clamped trilinear lookup (MacGridSampler3D.cpp:6-11 and the
@@ -60,15 +85,15 @@ struct Bracket {
 };
 
 template <bool STAGGERED, bool POW2 = false>
-__device__ __forceinline__ Bracket bracket(float coord, float h, int n, float ih = 0.f) {
+__device__ __forceinline__ Bracket bracket(float coord, const CellSize& c, int n) {
     Bracket b;
     if (STAGGERED) {
-        const float g = clampf_ref(div_h<POW2>(coord, h, ih), 0.f, float(n));
+        const float g = clampf_ref(div_h<POW2>(coord, c), 0.f, float(n));
         b.i0 = min(int(g), n - 1);
         b.i1 = b.i0 + 1;
         b.t = g - float(b.i0);
     } else {
-        const float g = clampf_ref(div_h<POW2>(coord, h, ih) - 0.5f, 0.f, float(n - 1));
+        const float g = clampf_ref(div_h<POW2>(coord, c) - 0.5f, 0.f, float(n - 1));
         b.i0 = int(g);
         b.i1 = min(b.i0 + 1, n - 1);
         b.t = g - float(b.i0);
@@ -110,11 +135,11 @@ __device__ __forceinline__ float sample_at(const float* __restrict__ f, int n, c
 // Trilinear sample of a field at location LOC, world position (px,py,pz), with
 // the reference's fixed 8-term order and left-to-right products.
 template <int LOC, bool POW2 = false>
-__device__ __forceinline__ float sample(const float* __restrict__ f, int n, float h, float px, float py,
-                                        float pz, float ih = 0.f) {
-    const Bracket bx = bracket<LOC == FACE_X, POW2>(px, h, n, ih);
-    const Bracket by = bracket<LOC == FACE_Y, POW2>(py, h, n, ih);
-    const Bracket bz = bracket<LOC == FACE_Z, POW2>(pz, h, n, ih);
+__device__ __forceinline__ float sample(const float* __restrict__ f, int n, const CellSize& c, float px, float py,
+                                        float pz) {
+    const Bracket bx = bracket<LOC == FACE_X, POW2>(px, c, n);
+    const Bracket by = bracket<LOC == FACE_Y, POW2>(py, c, n);
+    const Bracket bz = bracket<LOC == FACE_Z, POW2>(pz, c, n);
     return sample_at<LOC>(f, n, bx, by, bz);
 }
 
@@ -146,13 +171,12 @@ struct Vel {
 // MacGridSampler3D::velocity (MacGridSampler3D.cpp:73-75). The three
 // components share their brackets: per axis one staggered (the component
 // along it) and one centred (the other two).
-template <bool POW2 = false>
 __device__ __forceinline__ Vel velocity_at(const float* __restrict__ u, const float* __restrict__ v,
-                                           const float* __restrict__ w, int n, float h, float px, float py,
-                                           float pz, float ih = 0.f) {
-    const Bracket sx = bracket<true, POW2>(px, h, n, ih), cx = bracket<false, POW2>(px, h, n, ih);
-    const Bracket sy = bracket<true, POW2>(py, h, n, ih), cy = bracket<false, POW2>(py, h, n, ih);
-    const Bracket sz = bracket<true, POW2>(pz, h, n, ih), cz = bracket<false, POW2>(pz, h, n, ih);
+                                           const float* __restrict__ w, int n, const CellSize& c, float px, float py,
+                                           float pz) {
+    const Bracket sx = bracket<true>(px, c, n), cx = bracket<false>(px, c, n);
+    const Bracket sy = bracket<true>(py, c, n), cy = bracket<false>(py, c, n);
+    const Bracket sz = bracket<true>(pz, c, n), cz = bracket<false>(pz, c, n);
     Vel r;
     r.x = sample_at<FACE_X>(u, n, sx, cy, cz);
     r.y = sample_at<FACE_Y>(v, n, cx, sy, cz);
@@ -180,23 +204,73 @@ __device__ __forceinline__ Bracket bracket_half(int k, int n, bool staggered) {
     return b;
 }
 
-// velocity_at at the sample point of location LOC's node (x, y, z), for a
-// power-of-two cell size: the same values from integer brackets.
-template <int LOC>
-__device__ __forceinline__ Vel velocity_at_node(const float* __restrict__ u, const float* __restrict__ v,
-                                                const float* __restrict__ w, int n, int x, int y, int z) {
-    const int kx = 2 * x + (LOC == FACE_X ? 0 : 1);
-    const int ky = 2 * y + (LOC == FACE_Y ? 0 : 1);
-    const int kz = 2 * z + (LOC == FACE_Z ? 0 : 1);
-    const Bracket sx = bracket_half(kx, n, true), cx = bracket_half(kx, n, false);
-    const Bracket sy = bracket_half(ky, n, true), cy = bracket_half(ky, n, false);
-    const Bracket sz = bracket_half(kz, n, true), cz = bracket_half(kz, n, false);
-    Vel r;
-    r.x = sample_at<FACE_X>(u, n, sx, cy, cz);
-    r.y = sample_at<FACE_Y>(v, n, cx, sy, cz);
-    r.z = sample_at<FACE_Z>(w, n, cx, cy, sz);
-    return r;
+// The brackets of a node's velocity along one axis: staggered (the component
+// along it) and centred (the other two). They depend on the node's index alone.
+struct NodeAxis {
+    Bracket s, c;
+};
+template <bool STAGGERED, bool POW2>
+__device__ __forceinline__ NodeAxis node_axis(int i, const CellSize& c, int n) {
+    NodeAxis a;
+    if (POW2) {
+        const int k = 2 * i + (STAGGERED ? 0 : 1);
+        a.s = bracket_half(k, n, true);
+        a.c = bracket_half(k, n, false);
+    } else {
+        const float p = STAGGERED ? float(i) * c.h : (float(i) + 0.5f) * c.h;
+        a.s = bracket<true, false>(p, c, n);
+        a.c = bracket<false, false>(p, c, n);
+    }
+    return a;
 }
+
+// One component's trilinear lookups at the nodes of a column (x and y fixed,
+// plane after plane): the corner values of a plane with their products along x
+// and y serve the node below and the node above it, so a node costs one plane's
+// 4 loads in the place of 8. Products and sum in the order of trilinear().
+template <int LOC>
+struct ColumnSample {
+    int at[4];              // offsets of the corners in a plane
+    float wx[2], wy[2];     // 1 - t and t along x and y
+    float upper[4];         // products of plane `held`
+    int held;
+
+    __device__ __forceinline__ void start(int n, const Bracket& bx, const Bracket& by) {
+        const int ex = n + (LOC == FACE_X);
+        at[0] = ex * by.i0 + bx.i0;
+        at[1] = ex * by.i0 + bx.i1;
+        at[2] = ex * by.i1 + bx.i0;
+        at[3] = ex * by.i1 + bx.i1;
+        wx[0] = 1.f - bx.t;
+        wx[1] = bx.t;
+        wy[0] = 1.f - by.t;
+        wy[1] = by.t;
+        held = -1;
+    }
+    __device__ __forceinline__ void load(const float* __restrict__ f, int n, int z, float (&p)[4]) const {
+        const int base = (n + (LOC == FACE_X)) * (n + (LOC == FACE_Y)) * z;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) p[k] = __ldg(f + (base + at[k])) * wx[k & 1] * wy[k >> 1];
+    }
+    __device__ __forceinline__ float next(const float* __restrict__ f, int n, const Bracket& bz) {
+        float lower[4];
+        if (bz.i0 == held) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) lower[k] = upper[k];
+        } else {
+            load(f, n, bz.i0, lower);
+        }
+        load(f, n, bz.i1, upper);
+        held = bz.i1;
+        const float uz = 1.f - bz.t, tz = bz.t;
+        float s = lower[0] * uz;
+#pragma unroll
+        for (int k = 1; k < 4; ++k) s = s + lower[k] * uz;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s = s + upper[k] * tz;
+        return s;
+    }
+};
 
 // ---- reductions -------------------------------------------------------------
 

@@ -115,7 +115,7 @@ extern "C" __attribute__((visibility("default"))) vapor_status vapor_advect_noal
         float* scratch = scratch_for_current_context();
         const vb::Grid g{n, box, box / float(n)};
         vb::launch_advect(g, loc, dt, cfl_limit, method == VAPOR_MACCORMACK, source, flow_u, flow_v, flow_w, scratch,
-                          output, 1.f, static_cast<cudaStream_t>(stream));
+                          output, 1.f, nullptr, static_cast<cudaStream_t>(stream));
         VB_CUDA(cudaGetLastError());
     });
 }
