@@ -465,23 +465,23 @@ def main():
         launch time. One red+black iteration reads x and b and writes x,
         12 B/cell, so a one-colour launch is charged half of that, 6 B/cell
         (the other colour's half of x, written by the previous launch, is
-        mostly read back from L2); a temporally blocked launch of several
-        iterations reads x and b and writes x once, 12 B/cell. In the FPCG
-        preconditioner the last sweep of each CG step (`dot_launches` of
-        them) also reads r of the other colour and q of both, 6 B/cell
-        more."""
+        mostly read back from L2); a pass of two iterations reads x and b
+        and writes x once, 12 B/cell. In the FPCG preconditioner the last
+        colour sweep of each CG step (`dot_launches` of them) also reads r of
+        the other colour and q of both, 6 B/cell more; of its two passes one
+        starts from zero (8 B/cell) and one reads q, too (16): 12 again."""
         sor = ph["sor"]
         launches = max(1, sor["launches"])
         launch_ms = sor["ms"] / launches
         per_launch = sweeps / launches
         blocked = per_launch >= 1.5
-        nbytes = (12.0 if blocked else 6.0) * cells * (1.0 + dot_launches / launches)
+        nbytes = 12.0 * cells if blocked else 6.0 * cells * (1.0 + dot_launches / launches)
         achieved = nbytes / (launch_ms * 1e-3) / 1e9
-        line = {"bound": "hbm", "kernel": (f"k_sor_blocked ({per_launch:.0f} red+black iterations per launch)"
+        line = {"bound": "hbm", "kernel": (f"k_sor_wave ({per_launch:.0f} red+black iterations per launch)"
                                            if blocked else "k_sor_rbz (red-black colour sweep)"),
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_kind": peak_kind, "traffic": None if blocked else SOR_TRAFFIC_256 * cells / 256 ** 3,
-                "traffic_note": ("see profiles/ for the blocked sweep's ncu traffic" if blocked else
+                "traffic_note": ("see profiles/ for the ncu traffic of a pass" if blocked else
                                  "dram bytes read + written per launch from an ncu --set full capture at 256^3, "
                                  "scaled by cells for other sizes"),
                 "bytes_per_launch": nbytes, "avg_launch_us": launch_ms * 1e3,
