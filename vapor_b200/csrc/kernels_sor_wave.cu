@@ -22,12 +22,13 @@
 // All four half sweeps of a step meet a row with the same parity s, and a warp's
 // rows have one parity (kept together in shared memory too), so a warp runs code
 // in which the x neighbours, the wall slots and the ring positions are fixed:
-// some 250 instructions a step for 16 cell updates. A warp arrives at the
+// some 300 instructions a step for 16 cell updates. A warp arrives at the
 // rendezvous once it has loaded what half sweep 4 needs and waits for it before
-// it publishes half sweep 1, so half of a step runs while others are behind.
+// it publishes half sweep 1 (the warps that fetch wait first), so half of a step
+// runs while others are behind.
 //
-// Bound by shared memory (1600 wavefronts of 2500 cycles a step; the L1 pipe is
-// 70% busy) with issue at 55%, no longer by DRAM (36%). Measured, staged mixed
+// Bound by shared memory (1760 wavefronts of 2690 cycles a step; the L1 pipe is
+// 74% busy) and issue (65%), no longer by DRAM (39%): 62.8 us a pass at 256^3. Measured, staged mixed
 // projection, per iteration in all, one-colour launches against this pass: 136^3
 // 19.1 / 16.4 us, 160^3 23.0 / 18.6, 192^3 31.7 / 22.8, 224^3 47.2 / 31.1, 256^3
 // 58.0 / 38.3 (of which the sweeps 46 / 31). Moving the planes with 8-byte
@@ -197,7 +198,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_sor_wave(const __grid_constant_
     }
     // One half sweep of this thread's 4 slots in a plane, in two parts: what
     // comes from shared memory (c: the other colour of the plane) ...
-    auto load = [&](auto parity, const float* rhs, const float* c, const float (&o)[4], Near& m) {
+    auto load = [&](auto parity, const float* rhs, const float* c, Near& m) {
         constexpr int s = decltype(parity)::value;
         m.edge = s ? c[mine + 4] : c[mine - 1];
         ld4(c + ym_at, m.ym);
@@ -279,30 +280,31 @@ __global__ void __launch_bounds__(kThreads, 1) k_sor_wave(const __grid_constant_
         const bool live1 = there && sweeps > 0 && in(tau - 1, 3);
         if (live1) {
             Near m;
-            load(P{}, plane(kBA + K), plane(kXB + ((K + 3) & 3)), B1, m);
+            load(P{}, plane(kBA + K), plane(kXB + ((K + 3) & 3)), m);
             relax(P{}, No{}, tau - 1, A1, m, B1, B2, B0);
         }
         if (!fetcher_warp) gate();
         if (there) {
-        if (live1) st4(pub + mine, A1);
-        // 2: second colour in plane tau - 2, between A planes tau - 3 and tau - 1
-        if (sweeps > 0 && in(tau - 2, 2)) {
-            Near m;
-            load(P{}, plane(kBB + K), before, A2, m);
+            if (live1) st4(pub + mine, A1);
+            // 2: second colour in plane tau - 2, between A planes tau - 3 and tau - 1
+            if (sweeps > 0 && in(tau - 2, 2)) {
+                Near m;
+                load(P{}, plane(kBB + K), before, m);
                 relax(P{}, No{}, tau - 2, B2, m, A2, A3, A1);
                 st4(pub + 2 * kPlane + mine, B2);
-        }
-        // 3: first colour in plane tau - 3, between B planes tau - 4 and tau - 2
-        if (sweeps > 1 && in(tau - 3, 1)) {
-            Near m;
-            load(P{}, plane(kBA + ((K + 2) & 3)), before + 2 * kPlane, B3, m);
+            }
+            // 3: first colour in plane tau - 3, between B planes tau - 4 and tau - 2
+            if (sweeps > 1 && in(tau - 3, 1)) {
+                Near m;
+                load(P{}, plane(kBA + ((K + 2) & 3)), before + 2 * kPlane, m);
                 relax(P{}, No{}, tau - 3, A3, m, B3, B4, B2);
                 st4(pub + 4 * kPlane + mine, A3);
-            if (DOT && own && in(tau - 3, 0)) dot(A3, m.b, cA, tau - 3);
+                if (DOT && own && in(tau - 3, 0)) dot(A3, m.b, cA, tau - 3);
+            }
         }
-        }
+        // 4: second colour in plane tau - 4, between A planes tau - 5 and tau - 3
         Near m;
-        load(P{}, plane(kBB + ((K + 2) & 3)), before + 4 * kPlane, A4, m);
+        load(P{}, plane(kBB + ((K + 2) & 3)), before + 4 * kPlane, m);
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(go);
         if (there && in(tau - 4, 0)) {
