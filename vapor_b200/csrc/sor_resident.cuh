@@ -213,6 +213,10 @@ __global__ void __launch_bounds__(max_threads(PZ), 1) k_sor_resident(Args a) {
         asm volatile("mov.u32 %0, %%cluster_nctaid.x;\n" : "=r"(ctas));
     }
     if (ctrl->done) return;  // the same for every CTA
+    // Read before the CTAs' first rendezvous: the first CTA's last writes to the
+    // control block come after it, and nothing else orders a short fixed budget's
+    // end there against the start of a CTA far away.
+    const int max_iterations = ctrl->max_iterations, start_iterations = ctrl->iterations;
     const int n = a.n, row = a.row, G = a.groups;
     const int yblocks = GRID ? a.yblocks : 1;
     const int ybase = n / yblocks, yrem = n - ybase * yblocks;
@@ -566,9 +570,7 @@ __global__ void __launch_bounds__(max_threads(PZ), 1) k_sor_resident(Args a) {
     };
 
     const bool first_cta = rank == 0 && yb == 0;
-    const int max_iterations = ctrl->max_iterations;
-    int iterations = ctrl->iterations;
-    const int start_iterations = iterations;
+    int iterations = start_iterations;
     if (MODE == kFixed) {
         for (int it = iterations; it < max_iterations; ++it) {
             half_sweep(C0{}, No{});
