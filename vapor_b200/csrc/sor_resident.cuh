@@ -84,21 +84,24 @@ __device__ __forceinline__ void send4_global(unsigned char* to, int second, cons
                  "l"(pack2(v[2], __uint_as_float(epoch))), "l"(pack2(v[3], __uint_as_float(epoch)))
                  : "memory");
 }
+// The 4 words of such a pair of stores: loads of the width of a word, so that a
+// value and the number beside it are one access (elements of a vector access
+// are separate ones in the PTX memory model).
 struct Words {
-    uint32_t v[4], e[4];
+    pair_t w[4];
+    __device__ __forceinline__ uint4 values() const {
+        return make_uint4(uint32_t(w[0]), uint32_t(w[1]), uint32_t(w[2]), uint32_t(w[3]));
+    }
+    __device__ __forceinline__ bool complete(uint32_t epoch) const {
+        return uint32_t(w[0] >> 32) == epoch && uint32_t(w[1] >> 32) == epoch && uint32_t(w[2] >> 32) == epoch &&
+               uint32_t(w[3] >> 32) == epoch;
+    }
 };
-__device__ __forceinline__ void load_words(const unsigned char* from, int second, Words& w) {
-    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];\n"
-                 : "=r"(w.v[0]), "=r"(w.e[0]), "=r"(w.v[1]), "=r"(w.e[1])
-                 : "l"(from)
-                 : "memory");
-    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];\n"
-                 : "=r"(w.v[2]), "=r"(w.e[2]), "=r"(w.v[3]), "=r"(w.e[3])
-                 : "l"(from + second)
-                 : "memory");
+__device__ __forceinline__ void load_global(const unsigned char* from, pair_t& a, pair_t& b) {
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];\n" : "=l"(a), "=l"(b) : "l"(from) : "memory");
 }
-__device__ __forceinline__ bool complete(const Words& w, uint32_t epoch) {
-    return w.e[0] == epoch && w.e[1] == epoch && w.e[2] == epoch && w.e[3] == epoch;
+__device__ __forceinline__ void load_shared(uint32_t from, pair_t& a, pair_t& b) {
+    asm volatile("ld.relaxed.cluster.shared::cta.v2.b64 {%0, %1}, [%2];\n" : "=l"(a), "=l"(b) : "r"(from) : "memory");
 }
 
 __device__ __forceinline__ void ld4(const float* p, float (&o)[4]) {
@@ -124,17 +127,11 @@ __device__ __forceinline__ void send4(uint32_t addr, uint32_t second, const floa
 // false when the wait ran out.
 __device__ __forceinline__ bool receive4(uint32_t addr, uint32_t second, float* to, uint32_t epoch) {
     for (int i = 0; i < kPollLimit; ++i) {
-        uint32_t v[4], e[4];
-        asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n"
-                     : "=r"(v[0]), "=r"(e[0]), "=r"(v[1]), "=r"(e[1])
-                     : "r"(addr)
-                     : "memory");
-        asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n"
-                     : "=r"(v[2]), "=r"(e[2]), "=r"(v[3]), "=r"(e[3])
-                     : "r"(addr + second)
-                     : "memory");
-        if (e[0] == epoch && e[1] == epoch && e[2] == epoch && e[3] == epoch) {
-            *reinterpret_cast<uint4*>(to) = make_uint4(v[0], v[1], v[2], v[3]);
+        Words w;
+        load_shared(addr, w.w[0], w.w[1]);
+        load_shared(addr + second, w.w[2], w.w[3]);
+        if (w.complete(epoch)) {
+            *reinterpret_cast<uint4*>(to) = w.values();
             return true;
         }
     }
@@ -338,10 +335,11 @@ __global__ void __launch_bounds__(max_threads(PZ), 1) k_sor_resident(Args a) {
             const int second = tid + q * threads < 2 * per_block ? int(half_bytes) : y_half;
             Words w;
             for (int i = 0; !dead; ++i) {
-                load_words(a.words + from + c * 2 * second, second, w);
-                if (complete(w, epoch)) {
-                    *reinterpret_cast<uint4*>(s_x + c * colour_stride + s_i[table_at + 5 + 2 * q]) =
-                        make_uint4(w.v[0], w.v[1], w.v[2], w.v[3]);
+                const unsigned char* const at = a.words + from + c * 2 * second;
+                load_global(at, w.w[0], w.w[1]);
+                load_global(at + second, w.w[2], w.w[3]);
+                if (w.complete(epoch)) {
+                    *reinterpret_cast<uint4*>(s_x + c * colour_stride + s_i[table_at + 5 + 2 * q]) = w.values();
                     break;
                 }
                 if (i == kPollLimit) dead = true;
@@ -535,15 +533,12 @@ __global__ void __launch_bounds__(max_threads(PZ), 1) k_sor_resident(Args a) {
             }
             unsigned long long most = 0ull, any = 0ull;
             for (int r = tid; r < all; r += threads) {
-                uint32_t lo = 0, hi = 0, e0 = 0, e1 = 0;
-                for (int i = 0; (e0 != epoch || e1 != epoch) && !dead; ++i) {
-                    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];\n"
-                                 : "=r"(lo), "=r"(e0), "=r"(hi), "=r"(e1)
-                                 : "l"(red + size_t(r) * 16)
-                                 : "memory");
+                pair_t lo = 0, hi = 0;  // half of the result and the number each
+                for (int i = 0; (uint32_t(lo >> 32) != epoch || uint32_t(hi >> 32) != epoch) && !dead; ++i) {
+                    load_global(red + size_t(r) * 16, lo, hi);
                     if (i == kPollLimit) dead = true;
                 }
-                const unsigned long long v = (static_cast<unsigned long long>(hi) << 32) | lo;
+                const unsigned long long v = (hi << 32) | uint32_t(lo);
                 any |= v & (1ull << 63);
                 const unsigned long long u = v & ~(1ull << 63);
                 most = most < u ? u : most;
