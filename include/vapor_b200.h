@@ -368,6 +368,12 @@ vapor_status vapor_stage_advect_scalar_device(vapor_stage *stage, float dt, floa
 /* Pressure solver used by vapor_stage_project (vapor_solver_kind); the default
  * is VAPOR_SOLVER_RED_BLACK_SOR, the reference's SOR. */
 vapor_status vapor_stage_set_solver_kind(vapor_stage *stage, int32_t kind);
+/* Test hook for the pressure sweeps' bounded waits (no reference counterpart):
+ * with polls > 0, the first wait of every sweep launch of later projections
+ * polls for something that never comes that many times, runs out, and the
+ * projection returns VAPOR_RUNTIME_ERROR ("timed out"); 0 restores normal
+ * waits. The next projection starts clean. */
+vapor_status vapor_stage_set_wait_probe(vapor_stage *stage, int32_t polls);
 /* Solid obstacles for vapor_stage_project (extension, no reference
  * counterpart; Vapor's solvers have walls only). `mask` is n^3 host bytes,
  * x fastest, nonzero = solid; NULL removes the obstacles. Faces touching a

@@ -485,6 +485,7 @@ void Workspace::project(const float* ui, const float* vi, const float* wi, float
                         const vapor_linear_solve_options& o, int solver_kind, unet::UNet* warm,
                         unet::UNet* coarse, const float* rhs_field) {
     ProjectionArgs a{grid(), dt, omega, diagonal_floor, o};
+    a.wait_probe = wait_probe_;
     if (fluid_ > 0.0) {
         if (solver_kind != VAPOR_SOLVER_MIXED_REFINEMENT && solver_kind != VAPOR_SOLVER_FPCG)
             fail(VAPOR_INVALID_ARGUMENT,

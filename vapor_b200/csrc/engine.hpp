@@ -162,6 +162,7 @@ public:
         capturing_ = on;
         shared_device_ = shared;
     }
+    void set_wait_probe(int polls) { wait_probe_ = polls; }  // test hook, see ProjectionArgs
 
 private:
     void project_fpcg(const ProjectionArgs& a, unet::UNet* warm, unet::UNet* coarse, LoopCond cond,
@@ -201,6 +202,7 @@ private:
     Stream body_stream2_;               // records conditional bodies nested in a loop
     bool capturing_ = false;
     bool shared_device_ = false;        // recording one of several scenes that run together
+    int wait_probe_ = 0;
     long long total_iterations_ = 0;
     unsigned int sticky_errors_ = 0u;
     friend class Simulation;

@@ -128,6 +128,9 @@ struct ProjectionArgs {
     const uint8_t* diag = nullptr;
     const uint8_t* solid = nullptr;
     double fluid = 0.0;
+    // Test hook: > 0 makes the first wait of a sweep that waits poll for something
+    // that never comes, that many times, so that it runs out.
+    int wait_probe = 0;
 };
 // Graph while-loop control: when `active`, kernels that decide whether the
 // solve continues also set this conditional handle.

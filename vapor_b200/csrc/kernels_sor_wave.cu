@@ -64,6 +64,7 @@ constexpr int kSmem = (kPlanes * kPlane + kPad) * 4;
 constexpr int kHalf = kRows * kGroups;      // threads per row parity: 10 warps
 constexpr int kThreads = 2 * kHalf;
 constexpr int kWaitLimit = 1 << 20;
+constexpr int kDrainLimit = 1 << 14;
 
 struct WaveArgs {
     int n, hw;
@@ -76,6 +77,7 @@ struct WaveArgs {
     double* partials;        // DOT: 2 per CTA, z.b and z.q
     ProjControl* ctrl;
     int guarded, sweep_index;
+    int wait_probe;          // see ProjectionArgs
 };
 
 __device__ __forceinline__ void load_rows(uint32_t dst, const CUtensorMap* map, int x, int parity, int row, int z,
@@ -123,7 +125,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_sor_wave(const __grid_constant_
     extern __shared__ __align__(128) float s_mem[];
     __shared__ float s_max[32];
     __shared__ double s_sum[32];
-    __shared__ uint64_t s_full[2], s_go;
+    __shared__ uint64_t s_full[2], s_go, s_probe;
+    __shared__ int s_fetched[8];  // per fetching warp, the last step it fetched for
     const int n = a.n, hw = a.hw;
     int sweeps = 2;
     if (a.guarded) {
@@ -144,6 +147,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_sor_wave(const __grid_constant_
     const uint32_t smem = static_cast<uint32_t>(__cvta_generic_to_shared(s_mem));
     const uint32_t full = static_cast<uint32_t>(__cvta_generic_to_shared(s_full));
     const uint32_t go = static_cast<uint32_t>(__cvta_generic_to_shared(&s_go));
+    const uint32_t probe = static_cast<uint32_t>(__cvta_generic_to_shared(&s_probe));
     const int mine = odd * kBlock + kPad + r * kRow + 4 * g;          // this thread's slots in a plane
     const int ym_at = (odd ? mine - kBlock : mine + kBlock - kRow);   // rows before and behind: the other parity's
     const int yp_at = (odd ? mine - kBlock + kRow : mine + kBlock);
@@ -152,6 +156,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_sor_wave(const __grid_constant_
         tc::mbar_init(full, kLoads);
         tc::mbar_init(full + 8, kLoads);
         tc::mbar_init(go, kThreads / 32);
+        tc::mbar_init(probe, 1);
         tc::fence_mbarrier_init();
     }
     for (int i = tid; i < kPlanes * kPlane + kPad; i += kThreads) s_mem[i] = 0.f;
@@ -168,6 +173,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_sor_wave(const __grid_constant_
     const bool fetcher_warp = job < kLoads, fetcher = fetcher_warp && lane == 0;
     auto fetch = [&](int k) {
         if (!fetcher) return;
+        s_fetched[job] = k;
         const uint32_t bar = full + 8u * uint32_t(k & 1);
         const int lag = (job_array + 1) >> 1;  // 0, 1, 1, 2
         const int ring = job_array == 0 ? kXB + (k & 3) : (job_array == 1 ? kXA + (k & 1) : (job_array == 2 ? kBA : kBB) + (k & 3));
@@ -186,6 +192,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_sor_wave(const __grid_constant_
     float rmax = 0.f;
     double dzr = 0.0, dzq = 0.0;
     int limit = kWaitLimit;  // 0 once a wait has run out
+    if (a.wait_probe > 0 && !tc::mbar_wait(probe, 0u, a.wait_probe)) limit = 0;
     const long out = long(z0) * plane_floats + long(y) * hw + slot0;
     float* outA = a.xout + (there ? out + long(cA) * n * plane_floats : 0);
     float* outB = a.xout + (there ? out + long(cB) * n * plane_floats : 0);
@@ -264,7 +271,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_sor_wave(const __grid_constant_
         };
         if (fetcher_warp) {
             gate();
-            if (k + 1 < steps) fetch(k + 1);
+            if (k + 1 < steps && limit != 0) fetch(k + 1);
         }
         if (!tc::mbar_wait(full + 8 * (K & 1), uint32_t(k >> 1) & 1u, limit)) limit = 0;
         if (!FROM_ZERO) {
@@ -347,7 +354,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_sor_wave(const __grid_constant_
     };
     if ((odd + tau0 + 1 + cA) & 1) march(std::integral_constant<int, 1>{});
     else march(std::integral_constant<int, 0>{});
-    if (limit == 0) atomicOr(&a.ctrl->nonfinite, 8u);
+    if (limit == 0) {
+        atomicOr(&a.ctrl->nonfinite, 8u);
+        // Before the CTA's shared memory goes: the fetches of the last two steps
+        // may still be on their way. A fetcher begins one only after it has seen
+        // the barrier's one before it complete, so these are the phases to wait
+        // for (in vain, for the time of the limit, when another fetcher gave up).
+        if (fetcher && steps > 0)
+            for (int f = s_fetched[job]; f >= max(0, s_fetched[job] - 1); --f)
+                tc::mbar_wait(full + 8u * uint32_t(f & 1), uint32_t(f >> 1) & 1u, kDrainLimit);
+    }
     __syncthreads();
     if (RESID) {
         const float br = block_max(rmax, s_max);
@@ -455,6 +471,7 @@ WaveArgs make_args(const ProjectionArgs& p, const Plan& plan, int first, float* 
     for (int d = 0; d < 7; ++d) a.w[d] = p.omega / std::max(float(d), p.diagonal_floor);
     a.xout = xout;
     a.ctrl = ctrl;
+    a.wait_probe = p.wait_probe;
     return a;
 }
 
