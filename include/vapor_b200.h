@@ -636,6 +636,9 @@ vapor_status vapor_mac2d_refl_destroy(vapor_mac2d_refl *sim);
 vapor_status vapor_mac2d_refl_get_params(const vapor_mac2d_refl *sim, vapor_mac2d_refl_params *out);
 vapor_status vapor_mac2d_refl_set_params(vapor_mac2d_refl *sim, const vapor_mac2d_refl_params *params);
 vapor_status vapor_mac2d_refl_advance(vapor_mac2d_refl *sim, float dt);
+/* Test hook, as vapor_stage_set_wait_probe: the pressure sweeps' waits of later
+ * frames run out and the frame returns VAPOR_RUNTIME_ERROR. */
+vapor_status vapor_mac2d_refl_set_wait_probe(vapor_mac2d_refl *sim, int32_t polls);
 /* resetState(): zero fields, stirring stream back to the seed. */
 vapor_status vapor_mac2d_refl_reset(vapor_mac2d_refl *sim);
 /* Host arrays; any pointer may be NULL to skip it (pressure: download only). */

@@ -12,6 +12,9 @@ namespace vb {
 
 // Per-projection device state: reduction accumulators, loop control and the
 // assembled ProjectionResult. Lives in device memory, one per workspace.
+// Bits of ProjControl::nonfinite that end a solve at its next decision.
+constexpr unsigned int kSolveErrors = 4u | 8u;
+
 struct ProjControl {
     // accumulators, cleared at the start of a projection
     unsigned int div_before_bits;   // max |div| before, float bits

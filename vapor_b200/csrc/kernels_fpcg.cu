@@ -532,7 +532,7 @@ __global__ void k_cg_decide(ProjControl* ctrl, int use_if, cudaGraphConditionalH
     ctrl->res32_bits = 0u;
     const int recentre = double(rho) <= ctrl->target || double(rho) <= double(kRecentreDrop) * ctrl->r0 ||
                          ctrl->since >= kRecentreSweeps || ctrl->iterations >= ctrl->max_iterations ||
-                         (ctrl->nonfinite & 4u) != 0u;
+                         (ctrl->nonfinite & kSolveErrors) != 0u;
     ctrl->recentre = recentre;
     ctrl->result.linear_solve.iterations = ctrl->iterations;
     if (!recentre) ctrl->done = 0;

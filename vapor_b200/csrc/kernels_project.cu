@@ -613,7 +613,7 @@ __global__ void k_error_decide(ProjControl* ctrl, int sweeps, int use_conditiona
     ctrl->res32_bits = 0u;
     const int recentre = double(rho) <= ctrl->target || double(rho) <= double(kRecentreDrop) * ctrl->r0 ||
                          ctrl->since >= kRecentreSweeps || ctrl->iterations >= ctrl->max_iterations ||
-                         (ctrl->nonfinite & 4u) != 0u;
+                         (ctrl->nonfinite & kSolveErrors) != 0u;
     ctrl->recentre = recentre;
     if (use_if) cudaGraphSetConditional(if_handle, recentre ? 1u : 0u);
     ctrl->result.linear_solve.iterations = ctrl->iterations;
@@ -987,7 +987,7 @@ __global__ void k_check(ProjControl* ctrl, int iterations, int accumulate, int f
     ctrl->result.linear_solve.final_residual = res;
     ctrl->result.linear_solve.converged = converged;
     const int stop = (converged && !ctrl->fixed) || ctrl->iterations >= ctrl->max_iterations ||
-                     (ctrl->nonfinite & 4u) != 0u;
+                     (ctrl->nonfinite & kSolveErrors) != 0u;
     ctrl->done = stop;
     ctrl->continue_flag = !stop;
     if (use_conditional) cudaGraphSetConditional(handle, stop ? 0u : 1u);

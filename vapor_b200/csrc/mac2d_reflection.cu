@@ -311,7 +311,7 @@ __device__ __forceinline__ float divide_terms(float t, int terms) {
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) kr_sor_cluster(int n, int iterations, float omega, float h2, float dt,
                                                        const float* __restrict__ div, float* __restrict__ p,
-                                                       unsigned int* __restrict__ error) {
+                                                       unsigned int* __restrict__ error, int wait_probe) {
     using namespace resident;
     extern __shared__ __align__(16) float s_p[];  // [parity][rows + 2][row], then the halo words
     int rank, ctas;
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(THREADS) kr_sor_cluster(int n, int iterations,
             }
         }
     cluster_barrier();
-    bool dead = false;
+    bool dead = wait_probe > 0 && !receive4(words, second, s_p, kNever, wait_probe);
     if (link_lo) send4(to_lo + 2u * second, second, X[1], 1u);
     if (link_hi) send4(to_hi + 2u * second, second, X[1], 1u);
     const int yterms = int(y > 0) + int(y + 1 < n);
@@ -547,6 +547,7 @@ public:
     ~Mac2DReflection() { cudaStreamSynchronize(st_.s); }
 
     const vapor_mac2d_refl_params& params() const { return p_; }
+    void set_wait_probe(int polls) { wait_probe_ = polls; }  // test hook
     void set_params(const vapor_mac2d_refl_params& p) {
         p_ = p;
         patch_valid_ = false;
@@ -701,7 +702,8 @@ private:
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         VB_CUDA(cudaLaunchKernelEx(&cfg, rows * G <= 512 ? kr_sor_cluster<512> : kr_sor_cluster<1024>, n, iterations,
-                                   p_.sor_omega, h2, dt, static_cast<const float*>(div_.p), pressure_.p, error_.p));
+                                   p_.sor_omega, h2, dt, static_cast<const float*>(div_.p), pressure_.p, error_.p,
+                                   wait_probe_));
     }
 
     // project(dt, iterations) (:235-285).
@@ -745,6 +747,7 @@ private:
 
     int n_;
     vapor_mac2d_refl_params p_;
+    int wait_probe_ = 0;
     Stream st_;
     DevArray<float> smoke_, fwd_, back_, pressure_, div_, vx_, vy_, vxt_, vyt_, vxm_, vym_, vxh_, vyh_;
     DevArray<uint32_t> state_, special_;
@@ -831,6 +834,12 @@ VB_APIR vapor_status vapor_mac2d_refl_set_params(vapor_mac2d_refl* sim, const va
     return vb::guard([&] {
         require_r(sim && params, "null handle or parameters");
         sim->sim.set_params(*params);
+    });
+}
+VB_APIR vapor_status vapor_mac2d_refl_set_wait_probe(vapor_mac2d_refl* sim, int32_t polls) {
+    return vb::guard([&] {
+        require_r(sim && polls >= 0, "null handle or negative polls");
+        sim->sim.set_wait_probe(polls);
     });
 }
 VB_APIR vapor_status vapor_mac2d_refl_advance(vapor_mac2d_refl* sim, float dt) {

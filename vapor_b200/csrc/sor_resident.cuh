@@ -18,6 +18,7 @@ namespace resident {
 constexpr int kMaxCtas = 16;
 constexpr int kSmemLimit = 227 * 1024;
 constexpr int kPollLimit = 1 << 22;
+constexpr uint32_t kNever = 0xffffffffu;  // a number that no half sweep has
 
 using pair_t = unsigned long long;  // two floats
 
@@ -44,6 +45,7 @@ struct Args {
     int subtract_mean;
     int interval;            // sweeps per check
     int flag_nonfinite;      // mixed: a non-finite measured residual stops the solve
+    int wait_probe;          // see ProjectionArgs
 };
 
 // Threads per CTA: the registers that PZ planes of iterate, right-hand side
@@ -125,8 +127,9 @@ __device__ __forceinline__ void send4(uint32_t addr, uint32_t second, const floa
 }
 // Waits (bounded) until the 4 words carry `epoch`, then stores their values;
 // false when the wait ran out.
-__device__ __forceinline__ bool receive4(uint32_t addr, uint32_t second, float* to, uint32_t epoch) {
-    for (int i = 0; i < kPollLimit; ++i) {
+__device__ __forceinline__ bool receive4(uint32_t addr, uint32_t second, float* to, uint32_t epoch,
+                                         int limit = kPollLimit) {
+    for (int i = 0; i < limit; ++i) {
         Words w;
         load_shared(addr, w.w[0], w.w[1]);
         load_shared(addr + second, w.w[2], w.w[3]);
@@ -286,6 +289,21 @@ __global__ void __launch_bounds__(max_threads(PZ), 1) k_sor_resident(Args a) {
     const int total = 2 * colour_stride + (GRID ? 0 : 32 * per_block);
     for (int i = tid; i < total; i += threads) s_x[i] = 0.f;
     __syncthreads();
+    // a wait ran out: no further waits, the next check ends the solve and the
+    // error is reported at the end
+    bool dead = false;
+    if (a.wait_probe > 0) {
+        if (!GRID) {
+            dead = !receive4(words, half_bytes, s_x + row0, kNever, a.wait_probe);
+        } else {
+            Words w;
+            dead = true;
+            for (int i = 0; i < a.wait_probe && dead; ++i) {
+                load_global(a.words + size_t(blockIdx.x) * a.region, w.w[0], w.w[1]);
+                dead = uint32_t(w.w[0] >> 32) != kNever;
+            }
+        }
+    }
     const size_t rows = size_t(n) * n;
     float X[2][PZ][4], B[2][PZ][4];
     uint32_t D[2][PZ];  // mask_bytes
@@ -311,7 +329,6 @@ __global__ void __launch_bounds__(max_threads(PZ), 1) k_sor_resident(Args a) {
                 make_float4(X[c][k][0], X[c][k][1], X[c][k][2], X[c][k][3]);
         }
     if (!GRID) cluster_barrier();  // every CTA's halo words are cleared
-    bool dead = false;  // a wait ran out: no further waits, the error is reported at the end
     // one plane's updated slots to the neighbours that read them
     auto send = [&](int c, int k, bool bottom, bool top, const float (&v)[4], uint32_t epoch) {
         if (!GRID) {
@@ -493,7 +510,7 @@ __global__ void __launch_bounds__(max_threads(PZ), 1) k_sor_resident(Args a) {
     using C1 = std::integral_constant<int, 1>;
     int checks = 0;
     // the largest value over all CTAs (every thread gets it); keys order as the
-    // values; bit 63 of the result: some CTA saw `bad`
+    // values; bit 63 of the result: some CTA saw `bad` or a wait that ran out
     auto max_of_all = [&](unsigned long long key) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -501,12 +518,13 @@ __global__ void __launch_bounds__(max_threads(PZ), 1) k_sor_resident(Args a) {
             key = key < other ? other : key;
         }
         if (bad) atomicOr(&s_bad, 1);
+        if (dead) atomicOr(&s_dead, 1);
         if (lane == 0) s_warp[warp] = key;
         __syncthreads();
         auto block_result = [&]() {
             unsigned long long m = 0ull;
             for (int w = 0; w < (threads + 31) / 32; ++w) m = m < s_warp[w] ? s_warp[w] : m;
-            if (s_bad) m |= 1ull << 63;
+            if (s_bad || s_dead) m |= 1ull << 63;
             return m;
         };
         unsigned long long m = 0ull, flag = 0ull;
@@ -539,7 +557,7 @@ __global__ void __launch_bounds__(max_threads(PZ), 1) k_sor_resident(Args a) {
                     if (i == kPollLimit) dead = true;
                 }
                 const unsigned long long v = (hi << 32) | uint32_t(lo);
-                any |= v & (1ull << 63);
+                any |= dead ? 1ull << 63 : v & (1ull << 63);
                 const unsigned long long u = v & ~(1ull << 63);
                 most = most < u ? u : most;
             }
@@ -584,7 +602,7 @@ __global__ void __launch_bounds__(max_threads(PZ), 1) k_sor_resident(Args a) {
         }
     } else if (MODE == kMixed) {
         const double target = ctrl->target, drop = double(kRecentreDrop) * ctrl->r0;
-        const unsigned int nonfinite0 = ctrl->nonfinite & 4u;
+        const unsigned int nonfinite0 = ctrl->nonfinite & kSolveErrors;
         const int since0 = ctrl->since;
         bool stop = false;
         while (!stop) {
@@ -614,7 +632,7 @@ __global__ void __launch_bounds__(max_threads(PZ), 1) k_sor_resident(Args a) {
         if (!first_cta && tid == 0 && s_bad) atomicOr(&ctrl->nonfinite, 4u);
     } else {
         const double target = ctrl->target;
-        const unsigned int nonfinite0 = ctrl->nonfinite & 4u;
+        const unsigned int nonfinite0 = ctrl->nonfinite & kSolveErrors;
         double res = 0.0;
         bool stop = false;
         while (!stop) {
@@ -757,6 +775,7 @@ inline Args make_args(const ProjectionArgs& p, float* x, const float* b, ProjCon
     if (p.diag && a.hw % 4 == 0)
         for (int d = 0; d < 3; ++d) a.w[d] = a.w[3];
     a.interval = p.options.residual_check_interval;
+    a.wait_probe = p.wait_probe;
     return a;
 }
 
