@@ -335,6 +335,48 @@ def phase_rooflines(phases, steps, cells, peak, peak_kind):
     return out
 
 
+def sweep_roofline(ph, sweeps, cells, peak, peak_kind, dot_launches=0.0):
+    """The red-black sweep phase of one eager step covering `sweeps`
+    red+black iterations: per-launch algorithmic bytes over the average
+    launch time. One red+black iteration reads x and b and writes x,
+    12 B/cell, so a one-colour launch is charged half of that, 6 B/cell
+    (the other colour's half of x, written by the previous launch, is
+    mostly read back from L2); a pass of two iterations reads x and b
+    and writes x once, 12 B/cell. In the FPCG preconditioner the last
+    colour sweep of each CG step (`dot_launches` of them) also reads r of
+    the other colour and q of both, 6 B/cell more; of its two passes one
+    starts from zero (8 B/cell) and one reads q, too (16): 12 again.
+    The other forms run at most two iterations a launch and the resident
+    sweeps a whole check interval and more: these too read x and b and write
+    x once a launch, and what bounds them is the chain of half sweeps, not
+    those bytes."""
+    sor = ph["sor"]
+    launches = max(1, sor["launches"])
+    launch_ms = sor["ms"] / launches
+    per_launch = sweeps / launches
+    resident, passes = per_launch > 3.0, per_launch >= 1.5
+    nbytes = 12.0 * cells if passes else 6.0 * cells * (1.0 + dot_launches / launches)
+    achieved = nbytes / (launch_ms * 1e-3) / 1e9
+    if resident:
+        kernel = f"k_sor_resident ({per_launch:.0f} red+black iterations per launch)"
+    elif passes:
+        kernel = f"k_sor_wave ({per_launch:.0f} red+black iterations per launch)"
+    else:
+        kernel = "k_sor_rbz (red-black colour sweep)"
+    return {"bound": "latency" if resident else "hbm", "kernel": kernel,
+            "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+            "peak_kind": peak_kind, "traffic": None if passes else SOR_TRAFFIC_256 * cells / 256 ** 3,
+            "traffic_note": ("see profiles/ for the ncu traffic of a launch" if passes else
+                             "dram bytes read + written per launch from an ncu --set full capture at 256^3, "
+                             "scaled by cells for other sizes"),
+            "bytes_per_launch": nbytes, "avg_launch_us": launch_ms * 1e3,
+            "half_sweep_us": launch_ms * 1e3 / max(1e-9, 2.0 * per_launch),
+            "sweeps_per_s": sweeps / (sor["ms"] * 1e-3) if sor["ms"] > 0 else None,
+            "timing_note": "average launch time from CUDA events around the sweep phase of an eager replay of "
+                           "the benchmarked step on the simulation's stream (the kernels inside the step's "
+                           "CUDA graph cannot be bracketed one by one); launch gaps included"}
+
+
 def run_arm(vb, torch, args, n, fields, kind, net, dist, clocks=None):
     """Warm-up, then K timed steps (CUDA-graph replays) of one solver arm."""
     params = scene_params(vb.default_params(), n, args.rel, args.max_iterations, omega_for(n, args.omega),
@@ -459,38 +501,6 @@ def main():
     peak, peak_kind = measured_peaks()
     cells = n ** 3
 
-    def sor_roofline(ph, sweeps, dot_launches=0.0):
-        """The red-black sweep phase of one eager step covering `sweeps`
-        red+black iterations: per-launch algorithmic bytes over the average
-        launch time. One red+black iteration reads x and b and writes x,
-        12 B/cell, so a one-colour launch is charged half of that, 6 B/cell
-        (the other colour's half of x, written by the previous launch, is
-        mostly read back from L2); a pass of two iterations reads x and b
-        and writes x once, 12 B/cell. In the FPCG preconditioner the last
-        colour sweep of each CG step (`dot_launches` of them) also reads r of
-        the other colour and q of both, 6 B/cell more; of its two passes one
-        starts from zero (8 B/cell) and one reads q, too (16): 12 again."""
-        sor = ph["sor"]
-        launches = max(1, sor["launches"])
-        launch_ms = sor["ms"] / launches
-        per_launch = sweeps / launches
-        blocked = per_launch >= 1.5
-        nbytes = 12.0 * cells if blocked else 6.0 * cells * (1.0 + dot_launches / launches)
-        achieved = nbytes / (launch_ms * 1e-3) / 1e9
-        line = {"bound": "hbm", "kernel": (f"k_sor_wave ({per_launch:.0f} red+black iterations per launch)"
-                                           if blocked else "k_sor_rbz (red-black colour sweep)"),
-                "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "peak_kind": peak_kind, "traffic": None if blocked else SOR_TRAFFIC_256 * cells / 256 ** 3,
-                "traffic_note": ("see profiles/ for the ncu traffic of a pass" if blocked else
-                                 "dram bytes read + written per launch from an ncu --set full capture at 256^3, "
-                                 "scaled by cells for other sizes"),
-                "bytes_per_launch": nbytes, "avg_launch_us": launch_ms * 1e3,
-                "sweeps_per_s": sweeps / (sor["ms"] * 1e-3) if sor["ms"] > 0 else None,
-                "timing_note": "average launch time from CUDA events around the sweep phase of an eager replay of "
-                               "the benchmarked step on the simulation's stream (the kernels inside the step's "
-                               "CUDA graph cannot be bracketed one by one); launch gaps included"}
-        return line
-
     # Network (tensor cores): FLOPs of the coarse U-Net per application over
     # the coarse phase's time per application (restriction, normalization,
     # Galerkin scale and prolongation included, so this is a lower bound).
@@ -523,13 +533,15 @@ def main():
                   "value": aggregate_steps_per_second(world, args.steps, plain["ms"]), "unit": "steps/s",
                   "ms_per_step": plain["ms"] / args.steps, "sweeps_per_step": plain["iterations"],
                   "omega": omega_for(n, args.omega), "final_relative_residual": plain["final_relative_residual"],
-                  "converged": plain["converged"], "roofline": sor_roofline(plain_phases, plain_eager_sweeps),
+                  "converged": plain["converged"],
+                  "roofline": sweep_roofline(plain_phases, plain_eager_sweeps, cells, peak, peak_kind),
                   "phases_ms_per_step": {k: v["ms"] for k, v in plain_phases.items() if v["ms"] > 0}},
         "speedup_vs_plain": plain["ms"] / learned["ms"],
         "sweep_ratio_vs_plain": plain["iterations"] / max(1e-9, per_app * (learned["iterations"] + 2)),
         "gpu_launches": launches,
         "gpu_launches_note": "kernels per step counted on the eager replay of the same step, times steps",
-        "roofline": sor_roofline(phases, per_app * (eager_its + 2.0) * roof_steps, eager_its * roof_steps),
+        "roofline": sweep_roofline(phases, per_app * (eager_its + 2.0) * roof_steps, cells, peak, peak_kind,
+                                   eager_its * roof_steps),
         "roofline_tensor": {"bound": "tensor", "kernel": "coarse U-Net forward (k_conv3_zm and k_conv3_tc, 10 convolutions)",
                             "achieved": tflops, "peak": tpeak, "unit": "TFLOP/s", "frac": tflops / tpeak,
                             "peak_kind": "measured sustained", "flops_per_application": net_flops,
