@@ -146,9 +146,6 @@ vapor_phase_timings PhaseTimer::totals() {
 Workspace::Workspace(int n, float box, cudaStream_t stream)
     : n_(n), box_(box), stream_(stream), timer_(stream) {
     validate_grid(n, box);
-    configure_sor_cluster();
-    configure_sor_grid();
-    configure_sor_wave();
     const size_t faces = size_t(n) * n * (n + 1);
     const size_t slots = rb_count(n);  // red-black split storage
     b_.allocate(slots);

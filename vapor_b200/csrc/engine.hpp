@@ -5,6 +5,8 @@
 
 #include <cstdint>
 #include <functional>
+#include <mutex>
+#include <set>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -41,6 +43,25 @@ struct DevArray {
     void release();
     void zero(cudaStream_t s);
     size_t bytes() const { return n * sizeof(T); }
+};
+
+// Runs what a kernel needs before its first launch on a device (attributes for
+// its shared memory or cluster) once for each device.
+class OncePerDevice {
+public:
+    template <class F>
+    void operator()(F&& configure) {
+        int device = 0;
+        cuda_check(cudaGetDevice(&device), "cudaGetDevice");
+        std::lock_guard<std::mutex> lock(mutex_);
+        if (devices_.count(device)) return;
+        configure();
+        devices_.insert(device);
+    }
+
+private:
+    std::mutex mutex_;
+    std::set<int> devices_;
 };
 
 // Owning non-blocking CUDA stream.

@@ -177,9 +177,8 @@ int launch_sor_color_dot(const ProjectionArgs& a, int parity, float* x, const fl
 // - mean; _tolerance: the tolerance-driven solve on b - mean with its FP64
 // residual checks; _mixed: sweeps of the error equation up to the next
 // re-centring (ctrl->recentre = 1). A neighbour wait that runs out sets bit 3
-// of ctrl->nonfinite. configure_sor_cluster: once per device before any.
+// of ctrl->nonfinite.
 bool sor_cluster_applies(int n);
-void configure_sor_cluster();
 void launch_sor_cluster_fixed(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl, cudaStream_t s);
 void launch_sor_cluster_tolerance(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl,
                                   cudaStream_t s);
@@ -189,7 +188,6 @@ void launch_sor_cluster_mixed(const ProjectionArgs& p, float* e, const float* r3
 // 0 where it does not apply) are cleared; `compact` on the fewest SMs, for
 // scenes that share the device.
 size_t sor_grid_words(int n);
-void configure_sor_grid();
 void launch_sor_grid_fixed(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl, unsigned char* words,
                            bool compact, cudaStream_t s);
 void launch_sor_grid_tolerance(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl,
@@ -226,7 +224,6 @@ int sor_block_iterations(int n);
 // z.r and z.q when `q` is given (returns their block count, 0 when not written).
 bool sor_wave_applies(int n, bool masked);
 bool smooth_wave_applies(int n, bool masked);
-void configure_sor_wave();
 void launch_sor_wave(const ProjectionArgs& p, const float* xin, float* xout, const float* b, ProjControl* ctrl,
                      int sweep_index, bool measure, cudaStream_t s);
 void launch_smooth_wave_from_zero(const ProjectionArgs& p, float* z, const float* r, ProjControl* ctrl, cudaStream_t s);

@@ -46,13 +46,14 @@ struct Plan {
 };
 
 // Planes per thread as few as the threads allow, since they are updated one
-// after the other; then CTAs that divide n, so that no thread owns fewer; then
+// after the other (3 are never the fewest: 2 reach 48^3, from there 4 are
+// needed); then CTAs that divide n, so that no thread owns fewer; then
 // as many CTAs as the cluster allows.
 Plan plan_for(int n) {
     Plan best;
     if (n < 2) return best;
-    const int hwp = ((n + 1) / 2 + 3) / 4 * 4, G = hwp / 4;
-    for (int pz : {1, 2, 3, 4})
+    const int hwp = ((n + 1) / 2 + 3) / 4 * 4, G = hwp / 4, row = row_floats(hwp);
+    for (int pz : {1, 2, 4})
         for (bool divides : {true, false})
             for (int ctas = std::min(n, kMaxCtas); ctas >= 2; --ctas) {
                 const int slab = (n + ctas - 1) / ctas, blocks = (slab + pz - 1) / pz;
@@ -63,7 +64,7 @@ Plan plan_for(int n) {
                 p.pz = pz;
                 p.half = ((n + 1) / 2 * G + 31) / 32 * 32;
                 p.threads = 2 * p.half * blocks;
-                p.row = row_floats(hwp);
+                p.row = row;
                 p.planes = slab + 2;
                 p.smem = 2 * p.planes * (n + 2) * p.row * 4 + 8 * 2 * p.half * 16;
                 p.full = full;
@@ -72,56 +73,7 @@ Plan plan_for(int n) {
     return best;
 }
 
-template <int PZ, int MODE, int KIND, int GUARD>
-void configure_one() {
-    VB_CUDA(cudaFuncSetAttribute(k_sor_resident<PZ, MODE, KIND, GUARD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmemLimit - 2048));
-    VB_CUDA(cudaFuncSetAttribute(k_sor_resident<PZ, MODE, KIND, GUARD, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-}
-template <int PZ>
-void configure_planes() {
-    configure_one<PZ, kFixed, kUniform, 0>();
-    configure_one<PZ, kFixed, kUniform, 1>();
-    configure_one<PZ, kFixed, kUniform, 2>();
-    configure_one<PZ, kFixed, kGeneral, 2>();
-    configure_one<PZ, kTolerance, kUniform, 2>();
-    configure_one<PZ, kTolerance, kGeneral, 2>();
-    configure_one<PZ, kMixed, kUniform, 0>();
-    configure_one<PZ, kMixed, kUniform, 1>();
-    configure_one<PZ, kMixed, kUniform, 2>();
-    configure_one<PZ, kMixed, kGeneral, 2>();
-    configure_one<PZ, kMixed, kMasked, 2>();
-}
-
-template <int PZ, int MODE, int KIND, int GUARD>
-void launch_one(const Plan& p, const Args& a, cudaStream_t s) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned(p.ctas));
-    cfg.blockDim = dim3(unsigned(p.threads));
-    cfg.dynamicSmemBytes = size_t(p.smem);
-    cfg.stream = s;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = unsigned(p.ctas);
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    count_launch();
-    VB_CUDA(cudaLaunchKernelEx(&cfg, k_sor_resident<PZ, MODE, KIND, GUARD, false>, a));
-}
-
-template <int MODE, int KIND, int GUARD>
-void launch_kind(const Plan& p, const Args& a, cudaStream_t s) {
-    switch (p.pz) {
-        case 1: launch_one<1, MODE, KIND, GUARD>(p, a, s); break;
-        case 2: launch_one<2, MODE, KIND, GUARD>(p, a, s); break;
-        case 3: launch_one<3, MODE, KIND, GUARD>(p, a, s); break;
-        default: launch_one<4, MODE, KIND, GUARD>(p, a, s); break;
-    }
-}
-template <int MODE>
-void launch_mode(Args& a, cudaStream_t s) {
+void launch(Mode mode, Args& a, cudaStream_t s) {
     const Plan p = plan_for(a.n);
     a.row = p.row;
     a.planes = p.planes;
@@ -130,52 +82,39 @@ void launch_mode(Args& a, cudaStream_t s) {
     a.colour_stride = p.planes * a.plane;
     a.half_bytes = 2 * p.half * 16;
     // one weight and divisor when the floor is at or above the largest diagonal
-    const bool uniform = a.relax[3] == a.relax[6] && (MODE == kMixed || a.two_product);
+    const bool uniform = a.relax[3] == a.relax[6] && (mode == kMixed || a.two_product);
     const bool plain = a.hw % 4 == 0 && a.n % 2 == 0;
-    if constexpr (MODE == kMixed)
-        if (a.diag) return launch_kind<kMixed, kMasked, 2>(p, a, s);
-    if (!uniform) return launch_kind<MODE, kGeneral, 2>(p, a, s);
-    if constexpr (MODE != kTolerance) {
-        if (p.full && plain) return launch_kind<MODE, kUniform, 0>(p, a, s);
-        if (p.full) return launch_kind<MODE, kUniform, 1>(p, a, s);
+    const int kind = mode == kMixed && a.diag ? kMasked : (uniform ? kUniform : kGeneral);
+    const int guard = !p.full ? 2 : (plain ? 0 : 1);
+    const Shape shape{p.ctas, p.threads, p.smem};
+    switch (p.pz) {
+        case 1: launch_planes<1, false>(mode, kind, guard, shape, a, s); break;
+        case 2: launch_planes<2, false>(mode, kind, guard, shape, a, s); break;
+        default: launch_planes<4, false>(mode, kind, guard, shape, a, s); break;
     }
-    launch_kind<MODE, kUniform, 2>(p, a, s);
 }
 
 }  // namespace
 
 bool sor_cluster_applies(int n) { return plan_for(n).ctas > 0; }
 
-void configure_sor_cluster() {
-    static std::mutex mutex;
-    static std::set<int> devices;
-    int device = 0;
-    cuda_check(cudaGetDevice(&device), "cudaGetDevice");
-    std::lock_guard<std::mutex> lock(mutex);
-    if (!devices.insert(device).second) return;
-    configure_planes<1>();
-    configure_planes<2>();
-    configure_planes<3>();
-    configure_planes<4>();
-}
-
 void launch_sor_cluster_fixed(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl, cudaStream_t s) {
     Args a = make_args(p, x, b, ctrl);
     a.subtract_mean = 1;
-    launch_mode<kFixed>(a, s);
+    launch(kFixed, a, s);
 }
 
 void launch_sor_cluster_tolerance(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl,
                                   cudaStream_t s) {
     Args a = make_args(p, x, b, ctrl);
     a.subtract_mean = 1;
-    launch_mode<kTolerance>(a, s);
+    launch(kTolerance, a, s);
 }
 
 void launch_sor_cluster_mixed(const ProjectionArgs& p, float* e, const float* r32, ProjControl* ctrl, cudaStream_t s) {
     Args a = make_args(p, e, r32, ctrl);
     a.flag_nonfinite = a.hw % 4 != 0;  // as the separate residual pass of those sizes does
-    launch_mode<kMixed>(a, s);
+    launch(kMixed, a, s);
 }
 
 }  // namespace vb

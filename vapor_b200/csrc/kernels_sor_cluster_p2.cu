@@ -1,0 +1,8 @@
+// Resident sweeps in one cluster, 2 planes per thread.
+#include "sor_resident_launch.cuh"
+
+namespace vb {
+namespace resident {
+template void launch_planes<2, false>(Mode, int, int, const Shape&, const Args&, cudaStream_t);
+}
+}  // namespace vb

@@ -1,0 +1,8 @@
+// Resident sweeps in one cluster, 4 planes per thread.
+#include "sor_resident_launch.cuh"
+
+namespace vb {
+namespace resident {
+template void launch_planes<4, false>(Mode, int, int, const Shape&, const Args&, cudaStream_t);
+}
+}  // namespace vb

@@ -50,7 +50,7 @@ int device_sms() {
 Plan search_plan(int n, int sms, bool compact) {
     Plan best;
     if (n < 16) return best;
-    const int hwp = ((n + 1) / 2 + 3) / 4 * 4, G = hwp / 4;
+    const int hwp = ((n + 1) / 2 + 3) / 4 * 4, G = hwp / 4, row = row_floats(hwp);
     double least = 0.0;
     for (int yblocks = 1; yblocks <= n / 4; ++yblocks)
         for (int zblocks = 2; zblocks <= n && yblocks * zblocks <= sms; ++zblocks)
@@ -63,7 +63,7 @@ Plan search_plan(int n, int sms, bool compact) {
                 const int blocks = (slab + pz - 1) / pz;
                 p.half = ((rows + 1) / 2 * G + 31) / 32 * 32;
                 p.threads = 2 * p.half * blocks;
-                p.row = row_floats(hwp);
+                p.row = row;
                 p.planes = slab + 2;
                 p.plane = (rows + 2) * p.row;
                 p.smem = 2 * p.planes * p.plane * 4 + kTable * 4 * p.threads;
@@ -93,51 +93,7 @@ Plan plan_for(int n, bool compact) {
     return known[key] = search_plan(n, std::get<1>(key), compact);
 }
 
-template <int PZ, int MODE, int KIND, int GUARD>
-void configure_one() {
-    VB_CUDA(cudaFuncSetAttribute(k_sor_resident<PZ, MODE, KIND, GUARD, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit - 2048));
-}
-template <int PZ>
-void configure_planes() {
-    configure_one<PZ, kFixed, kUniform, 0>();
-    configure_one<PZ, kFixed, kUniform, 2>();
-    configure_one<PZ, kFixed, kGeneral, 2>();
-    configure_one<PZ, kTolerance, kUniform, 2>();
-    configure_one<PZ, kTolerance, kGeneral, 2>();
-    configure_one<PZ, kMixed, kUniform, 0>();
-    configure_one<PZ, kMixed, kUniform, 2>();
-    configure_one<PZ, kMixed, kGeneral, 2>();
-    configure_one<PZ, kMixed, kMasked, 2>();
-}
-
-template <int PZ, int MODE, int KIND, int GUARD>
-void launch_one(const Plan& p, const Args& a, cudaStream_t s) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned(p.ctas()));
-    cfg.blockDim = dim3(unsigned(p.threads));
-    cfg.dynamicSmemBytes = size_t(p.smem);
-    cfg.stream = s;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeCooperative;
-    attr.val.cooperative = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    count_launch();
-    VB_CUDA(cudaLaunchKernelEx(&cfg, k_sor_resident<PZ, MODE, KIND, GUARD, true>, a));
-}
-
-template <int MODE, int KIND, int GUARD>
-void launch_kind(const Plan& p, const Args& a, cudaStream_t s) {
-    switch (p.pz) {
-        case 1: launch_one<1, MODE, KIND, GUARD>(p, a, s); break;
-        case 2: launch_one<2, MODE, KIND, GUARD>(p, a, s); break;
-        case 3: launch_one<3, MODE, KIND, GUARD>(p, a, s); break;
-        default: launch_one<4, MODE, KIND, GUARD>(p, a, s); break;
-    }
-}
-template <int MODE>
-void launch_mode(Args& a, unsigned char* words, bool compact, cudaStream_t s) {
+void launch(Mode mode, Args& a, unsigned char* words, bool compact, cudaStream_t s) {
     const Plan p = plan_for(a.n, compact);
     a.row = p.row;
     a.planes = p.planes;
@@ -152,14 +108,17 @@ void launch_mode(Args& a, unsigned char* words, bool compact, cudaStream_t s) {
     a.words = words;
     VB_CUDA(cudaMemsetAsync(words, 0, p.bytes(), s));  // the numbers start anew
     // one weight and divisor when the floor is at or above the largest diagonal
-    const bool uniform = a.relax[3] == a.relax[6] && (MODE == kMixed || a.two_product);
+    const bool uniform = a.relax[3] == a.relax[6] && (mode == kMixed || a.two_product);
     const bool plain = a.hw % 4 == 0 && a.n % 2 == 0;
-    if constexpr (MODE == kMixed)
-        if (a.diag) return launch_kind<kMixed, kMasked, 2>(p, a, s);
-    if (!uniform) return launch_kind<MODE, kGeneral, 2>(p, a, s);
-    if constexpr (MODE != kTolerance)
-        if (p.full && plain) return launch_kind<MODE, kUniform, 0>(p, a, s);
-    launch_kind<MODE, kUniform, 2>(p, a, s);
+    const int kind = mode == kMixed && a.diag ? kMasked : (uniform ? kUniform : kGeneral);
+    const int guard = p.full && plain ? 0 : 2;
+    const Shape shape{p.ctas(), p.threads, p.smem};
+    switch (p.pz) {
+        case 1: launch_planes<1, true>(mode, kind, guard, shape, a, s); break;
+        case 2: launch_planes<2, true>(mode, kind, guard, shape, a, s); break;
+        case 3: launch_planes<3, true>(mode, kind, guard, shape, a, s); break;
+        default: launch_planes<4, true>(mode, kind, guard, shape, a, s); break;
+    }
 }
 
 }  // namespace
@@ -173,38 +132,25 @@ size_t sor_grid_words(int n) {
     return bytes;
 }
 
-void configure_sor_grid() {
-    static std::mutex mutex;
-    static std::set<int> devices;
-    int device = 0;
-    VB_CUDA(cudaGetDevice(&device));
-    std::lock_guard<std::mutex> lock(mutex);
-    if (!devices.insert(device).second) return;
-    configure_planes<1>();
-    configure_planes<2>();
-    configure_planes<3>();
-    configure_planes<4>();
-}
-
 void launch_sor_grid_fixed(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl, unsigned char* words,
                            bool compact, cudaStream_t s) {
     Args a = make_args(p, x, b, ctrl);
     a.subtract_mean = 1;
-    launch_mode<kFixed>(a, words, compact, s);
+    launch(kFixed, a, words, compact, s);
 }
 
 void launch_sor_grid_tolerance(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl,
                                unsigned char* words, bool compact, cudaStream_t s) {
     Args a = make_args(p, x, b, ctrl);
     a.subtract_mean = 1;
-    launch_mode<kTolerance>(a, words, compact, s);
+    launch(kTolerance, a, words, compact, s);
 }
 
 void launch_sor_grid_mixed(const ProjectionArgs& p, float* e, const float* r32, ProjControl* ctrl,
                            unsigned char* words, bool compact, cudaStream_t s) {
     Args a = make_args(p, e, r32, ctrl);
     a.flag_nonfinite = a.hw % 4 != 0;  // as the separate residual pass of those sizes does
-    launch_mode<kMixed>(a, words, compact, s);
+    launch(kMixed, a, words, compact, s);
 }
 
 }  // namespace vb

@@ -1,0 +1,8 @@
+// Resident sweeps in the whole device, 3 planes per thread.
+#include "sor_resident_launch.cuh"
+
+namespace vb {
+namespace resident {
+template void launch_planes<3, true>(Mode, int, int, const Shape&, const Args&, cudaStream_t);
+}
+}  // namespace vb

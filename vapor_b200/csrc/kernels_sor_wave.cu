@@ -454,6 +454,11 @@ CUtensorMap field_map(const float* field, int n, int rows) {
 
 template <bool FROM_ZERO, bool RESID, bool DOT>
 void launch(const Plan& p, const WaveArgs& a, const float* xin, const float* b, cudaStream_t s) {
+    static OncePerDevice once;
+    once([] {
+        VB_CUDA(cudaFuncSetAttribute(k_sor_wave<FROM_ZERO, RESID, DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     kSmem));
+    });
     const CUtensorMap bmap = field_map(b, a.n, a.rows);
     const CUtensorMap xmap = FROM_ZERO ? bmap : field_map(xin, a.n, a.rows);
     count_launch();
@@ -485,19 +490,6 @@ bool sor_wave_applies(int n, bool masked) { return !masked && n % 8 == 0 && n > 
 // passes: 17.0 / 17.2 ms at 160^3, 22.6 / 22.4 at 192^3, 31.7 / 30.2 at 224^3,
 // 42.8 / 39.8 at 256^3.
 bool smooth_wave_applies(int n, bool masked) { return n >= 192 && sor_wave_applies(n, masked); }
-
-void configure_sor_wave() {
-    static std::mutex mutex;
-    static std::set<int> devices;
-    int device = 0;
-    VB_CUDA(cudaGetDevice(&device));
-    std::lock_guard<std::mutex> lock(mutex);
-    if (!devices.insert(device).second) return;
-    VB_CUDA(cudaFuncSetAttribute(k_sor_wave<false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    VB_CUDA(cudaFuncSetAttribute(k_sor_wave<false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    VB_CUDA(cudaFuncSetAttribute(k_sor_wave<true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    VB_CUDA(cudaFuncSetAttribute(k_sor_wave<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-}
 
 void launch_sor_wave(const ProjectionArgs& p, const float* xin, float* xout, const float* b, ProjControl* ctrl,
                      int sweep_index, bool measure, cudaStream_t s) {

@@ -510,22 +510,6 @@ __global__ void kr_diagnostics(int n, float h, const float* __restrict__ vx, con
 
 // ---- host side ----
 
-// Shared-memory and cluster limits of the kernels, once per device.
-void configure_kernels() {
-    static std::mutex mutex;
-    static std::set<int> devices;
-    int device = 0;
-    VB_CUDA(cudaGetDevice(&device));
-    std::lock_guard<std::mutex> lock(mutex);
-    if (!devices.insert(device).second) return;
-    VB_CUDA(cudaFuncSetAttribute(kr_limit_march, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-    for (const void* kernel :
-         {reinterpret_cast<const void*>(kr_sor_cluster<512>), reinterpret_cast<const void*>(kr_sor_cluster<1024>)}) {
-        VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
-        VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    }
-}
-
 class Mac2DReflection {
 public:
     Mac2DReflection(int n, const vapor_mac2d_refl_params& p) : n_(n), p_(p) {
@@ -539,7 +523,6 @@ public:
         limit_.zero(st_.s);  // records of no cell stay zero
         energy_.allocate(1);
         maxima_.allocate(2);
-        configure_kernels();
         error_.allocate(1);
         error_.zero(st_.s);
         reset();
@@ -633,6 +616,7 @@ private:
         float4* const records = reinterpret_cast<float4*>(limit_.p);
         float* const marched = limit_.p + size_t(4) * warps * steps * 32;
         kr_limit_prepare<<<blocks_r(cells()), kT, 0, st_.s>>>(n_, smoke_.p, fwd_.p, back_.p, records, special_.p);
+        // at most 40 KB of shared memory (n = 512), within what needs no attribute
         kr_limit_march<<<1, warps * 32, size_t(warps) * (steps + 64) * sizeof(float), st_.s>>>(
             n_, records, special_.p, marched, smoke_.p, fwd_.p, back_.p);
         kr_scale<<<blocks_r(cells()), kT, 0, st_.s>>>(n_, decay, smoke_.p, marched, special_.p, smoke_.p);
@@ -701,7 +685,14 @@ private:
         attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        VB_CUDA(cudaLaunchKernelEx(&cfg, rows * G <= 512 ? kr_sor_cluster<512> : kr_sor_cluster<1024>, n, iterations,
+        static OncePerDevice once[2];
+        const bool small = rows * G <= 512;
+        const auto kernel = small ? kr_sor_cluster<512> : kr_sor_cluster<1024>;
+        once[small]([&] {
+            VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
+            VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        });
+        VB_CUDA(cudaLaunchKernelEx(&cfg, kernel, n, iterations,
                                    p_.sor_omega, h2, dt, static_cast<const float*>(div_.p), pressure_.p, error_.p,
                                    wait_probe_));
     }

@@ -751,6 +751,15 @@ inline int row_floats(int hwp) {
     return best;
 }
 
+// A launch: CTAs (of one cluster, or over the device), threads and bytes of
+// shared memory of each.
+struct Shape {
+    int ctas, threads, smem;
+};
+// Launches the kernel of this mode, kind and guard (sor_resident_launch.cuh).
+template <int PZ, bool GRID>
+void launch_planes(Mode mode, int kind, int guard, const Shape& p, const Args& a, cudaStream_t s);
+
 inline Args make_args(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl) {
     Args a{};
     a.n = p.g.n;
