@@ -519,8 +519,7 @@ public:
         for (DevArray<float>* a : {&vx_, &vy_, &vxt_, &vyt_, &vxm_, &vym_, &vxh_, &vyh_}) a->allocate(faces);
         state_.allocate(1);
         special_.allocate(1);
-        limit_.allocate(size_t(5) * ((n + 31) / 32) * march_steps(n) * 32);
-        limit_.zero(st_.s);  // records of no cell stay zero
+        if (p.mac_cormack_smoke) prepare_limiter();
         energy_.allocate(1);
         maxima_.allocate(2);
         error_.allocate(1);
@@ -557,6 +556,7 @@ public:
             !std::isfinite(p.stir_strength) || p.stir_strength < 0.f || !std::isfinite(p.sor_omega) ||
             p.sor_omega <= 0.f || p.sor_omega >= 2.f || p.project_iterations < 0)
             fail(VAPOR_INVALID_ARGUMENT, "Invalid 2D reflection step or parameters");
+        if (p.mac_cormack_smoke) prepare_limiter();
         walls(vx_.p, vy_.p);
         step(dt, p.buoyancy, std::exp(-p.smoke_decay / 60.f), p.source_strength, p.project_iterations);
         uint32_t error = 0;
@@ -602,6 +602,12 @@ private:
     long cells() const { return long(n_) * n_; }
     long faces() const { return long(n_) * (n_ + 1); }
     void walls(float* u, float* v) { kr_walls<<<blocks_r(n_), kT, 0, st_.s>>>(n_, u, v); }
+
+    void prepare_limiter() {
+        if (limit_.p) return;
+        limit_.allocate(size_t(5) * ((n_ + 31) / 32) * march_steps(n_) * 32);
+        limit_.zero(st_.s);  // records of no cell stay zero
+    }
 
     // advectScalar(smoke, dt) through the current velocity, then smoke *= decay.
     void advect_smoke(float dt, float decay) {
