@@ -374,6 +374,11 @@ vapor_status vapor_stage_set_solver_kind(vapor_stage *stage, int32_t kind);
  * projection returns VAPOR_RUNTIME_ERROR ("timed out"); 0 restores normal
  * waits. The next projection starts clean. */
 vapor_status vapor_stage_set_wait_probe(vapor_stage *stage, int32_t polls);
+
+/* Test hook: with 0 later projections run as on a device that cannot hold the
+ * kernels of the resident sweeps (one launch per colour in their place, the
+ * same results); 1 restores the choice. */
+vapor_status vapor_stage_set_resident_sweeps(vapor_stage *stage, int32_t enabled);
 /* Solid obstacles for vapor_stage_project (extension, no reference
  * counterpart; Vapor's solvers have walls only). `mask` is n^3 host bytes,
  * x fastest, nonzero = solid; NULL removes the obstacles. Faces touching a
@@ -639,6 +644,8 @@ vapor_status vapor_mac2d_refl_advance(vapor_mac2d_refl *sim, float dt);
 /* Test hook, as vapor_stage_set_wait_probe: the pressure sweeps' waits of later
  * frames run out and the frame returns VAPOR_RUNTIME_ERROR. */
 vapor_status vapor_mac2d_refl_set_wait_probe(vapor_mac2d_refl *sim, int32_t polls);
+/* Test hook, as vapor_stage_set_resident_sweeps. */
+vapor_status vapor_mac2d_refl_set_resident_sweeps(vapor_mac2d_refl *sim, int32_t enabled);
 /* resetState(): zero fields, stirring stream back to the seed. */
 vapor_status vapor_mac2d_refl_reset(vapor_mac2d_refl *sim);
 /* Host arrays; any pointer may be NULL to skip it (pressure: download only). */

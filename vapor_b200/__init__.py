@@ -112,6 +112,7 @@ def _declare(lib):
     f("vapor_stage_advect_scalar_device", _vp, C.c_float, C.c_float, C.c_int32, _vp, _vp, _vp, _vp)
     f("vapor_stage_set_solver_kind", _vp, C.c_int32)
     f("vapor_stage_set_wait_probe", _vp, C.c_int32)
+    f("vapor_stage_set_resident_sweeps", _vp, C.c_int32)
     f("vapor_stage_stream", _vp, C.POINTER(_vp))
     f("vapor_stage_set_solid", _vp, _vp)
     f("vapor_stage_solve_rhs", _vp, _vp, C.POINTER(ProjectionOptions), C.c_float, C.POINTER(ProjectionResult), _vp)

@@ -321,6 +321,9 @@ VB_API vapor_status vapor_stage_set_solver_kind(vapor_stage* stage, int32_t kind
 VB_API vapor_status vapor_stage_set_wait_probe(vapor_stage* stage, int32_t polls) {
     STAGE_GUARD(require(polls >= 0, "polls must be non-negative"); stage->stage.workspace().set_wait_probe(polls));
 }
+VB_API vapor_status vapor_stage_set_resident_sweeps(vapor_stage* stage, int32_t enabled) {
+    STAGE_GUARD(stage->stage.workspace().set_resident_sweeps(enabled != 0));
+}
 VB_API vapor_status vapor_stage_set_solid(vapor_stage* stage, const uint8_t* mask) {
     STAGE_GUARD(stage->stage.set_solid(mask));
 }

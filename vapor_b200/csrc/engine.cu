@@ -503,8 +503,15 @@ void Workspace::project(const float* ui, const float* vi, const float* wi, float
     // device: 1.2 / 1.7 us at 48^3; at 50^3 fixed budgets 2.1 / 1.6 and tolerance
     // checks 2.7 / 2.1, the mixed solver 1.8 / 1.9; at 64^3 1.9 / 1.4, 2.9 / 1.9
     // and 1.8 / 1.6.
-    const bool in_grid = sor_words_.p && (!sor_cluster_applies(n_) || (!mixed && !shared_device_));
-    const bool cluster = !fpcg && (in_grid || sor_cluster_applies(n_)) && sor_block_iterations(n_) == 0;
+    // Where the device cannot hold the one, the other runs, or launches per colour.
+    const bool resident = resident_sweeps_ && !fpcg && sor_block_iterations(n_) == 0;
+    const bool grid_first = !sor_cluster_applies(n_) || (!mixed && !shared_device_);
+    const SweepMode mode = mixed ? SweepMode::kMixed : (o.fixed_iterations ? SweepMode::kFixed : SweepMode::kTolerance);
+    auto grid_runs = [&] { return sor_words_.p && sor_grid_runs(a, mode, shared_device_); };
+    bool in_grid = resident && grid_first && grid_runs();
+    const bool in_cluster = resident && !in_grid && sor_cluster_runs(a, mode);
+    if (resident && !in_cluster && !grid_first) in_grid = grid_runs();
+    const bool cluster = in_grid || in_cluster;
     if (mixed) ensure_mixed();
     if (fpcg) ensure_fpcg(coarse != nullptr);
     // A device-side while loop is recorded only when the solve has one; a

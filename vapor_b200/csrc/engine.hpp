@@ -184,6 +184,7 @@ public:
         shared_device_ = shared;
     }
     void set_wait_probe(int polls) { wait_probe_ = polls; }  // test hook, see ProjectionArgs
+    void set_resident_sweeps(bool on) { resident_sweeps_ = on; }  // test hook: as on a device that cannot hold them
 
 private:
     void project_fpcg(const ProjectionArgs& a, unet::UNet* warm, unet::UNet* coarse, LoopCond cond,
@@ -224,6 +225,7 @@ private:
     bool capturing_ = false;
     bool shared_device_ = false;        // recording one of several scenes that run together
     int wait_probe_ = 0;
+    bool resident_sweeps_ = true;
     long long total_iterations_ = 0;
     unsigned int sticky_errors_ = 0u;
     friend class Simulation;

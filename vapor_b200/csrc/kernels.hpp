@@ -178,7 +178,10 @@ int launch_sor_color_dot(const ProjectionArgs& a, int parity, float* x, const fl
 // residual checks; _mixed: sweeps of the error equation up to the next
 // re-centring (ctrl->recentre = 1). A neighbour wait that runs out sets bit 3
 // of ctrl->nonfinite.
+// _runs: and the device can hold the launch (a partition of a GPU may not).
+enum class SweepMode { kFixed, kTolerance, kMixed };
 bool sor_cluster_applies(int n);
+bool sor_cluster_runs(const ProjectionArgs& p, SweepMode mode);
 void launch_sor_cluster_fixed(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl, cudaStream_t s);
 void launch_sor_cluster_tolerance(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl,
                                   cudaStream_t s);
@@ -188,6 +191,7 @@ void launch_sor_cluster_mixed(const ProjectionArgs& p, float* e, const float* r3
 // 0 where it does not apply) are cleared; `compact` on the fewest SMs, for
 // scenes that share the device.
 size_t sor_grid_words(int n);
+bool sor_grid_runs(const ProjectionArgs& p, SweepMode mode, bool compact);
 void launch_sor_grid_fixed(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl, unsigned char* words,
                            bool compact, cudaStream_t s);
 void launch_sor_grid_tolerance(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl,

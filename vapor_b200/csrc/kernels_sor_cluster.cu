@@ -73,7 +73,7 @@ Plan plan_for(int n) {
     return best;
 }
 
-void launch(Mode mode, Args& a, cudaStream_t s) {
+bool launch(Mode mode, Args& a, bool query, cudaStream_t s) {
     const Plan p = plan_for(a.n);
     a.row = p.row;
     a.planes = p.planes;
@@ -88,9 +88,9 @@ void launch(Mode mode, Args& a, cudaStream_t s) {
     const int guard = !p.full ? 2 : (plain ? 0 : 1);
     const Shape shape{p.ctas, p.threads, p.smem};
     switch (p.pz) {
-        case 1: launch_planes<1, false>(mode, kind, guard, shape, a, s); break;
-        case 2: launch_planes<2, false>(mode, kind, guard, shape, a, s); break;
-        default: launch_planes<4, false>(mode, kind, guard, shape, a, s); break;
+        case 1: return launch_planes<1, false>(mode, kind, guard, shape, a, query, s);
+        case 2: return launch_planes<2, false>(mode, kind, guard, shape, a, query, s);
+        default: return launch_planes<4, false>(mode, kind, guard, shape, a, query, s);
     }
 }
 
@@ -98,23 +98,29 @@ void launch(Mode mode, Args& a, cudaStream_t s) {
 
 bool sor_cluster_applies(int n) { return plan_for(n).ctas > 0; }
 
+bool sor_cluster_runs(const ProjectionArgs& p, SweepMode mode) {
+    if (!sor_cluster_applies(p.g.n)) return false;
+    Args a = make_args(p, nullptr, nullptr, nullptr);
+    return launch(Mode(mode), a, true, nullptr);
+}
+
 void launch_sor_cluster_fixed(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl, cudaStream_t s) {
     Args a = make_args(p, x, b, ctrl);
     a.subtract_mean = 1;
-    launch(kFixed, a, s);
+    launch(kFixed, a, false, s);
 }
 
 void launch_sor_cluster_tolerance(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl,
                                   cudaStream_t s) {
     Args a = make_args(p, x, b, ctrl);
     a.subtract_mean = 1;
-    launch(kTolerance, a, s);
+    launch(kTolerance, a, false, s);
 }
 
 void launch_sor_cluster_mixed(const ProjectionArgs& p, float* e, const float* r32, ProjControl* ctrl, cudaStream_t s) {
     Args a = make_args(p, e, r32, ctrl);
     a.flag_nonfinite = a.hw % 4 != 0;  // as the separate residual pass of those sizes does
-    launch(kMixed, a, s);
+    launch(kMixed, a, false, s);
 }
 
 }  // namespace vb

@@ -93,7 +93,7 @@ Plan plan_for(int n, bool compact) {
     return known[key] = search_plan(n, std::get<1>(key), compact);
 }
 
-void launch(Mode mode, Args& a, unsigned char* words, bool compact, cudaStream_t s) {
+bool launch(Mode mode, Args& a, unsigned char* words, bool compact, bool query, cudaStream_t s) {
     const Plan p = plan_for(a.n, compact);
     a.row = p.row;
     a.planes = p.planes;
@@ -106,7 +106,7 @@ void launch(Mode mode, Args& a, unsigned char* words, bool compact, cudaStream_t
     a.half_bytes = 2 * p.half * 16;
     a.y_half = (p.planes - 2) * a.groups * 16;
     a.words = words;
-    VB_CUDA(cudaMemsetAsync(words, 0, p.bytes(), s));  // the numbers start anew
+    if (!query) VB_CUDA(cudaMemsetAsync(words, 0, p.bytes(), s));  // the numbers start anew
     // one weight and divisor when the floor is at or above the largest diagonal
     const bool uniform = a.relax[3] == a.relax[6] && (mode == kMixed || a.two_product);
     const bool plain = a.hw % 4 == 0 && a.n % 2 == 0;
@@ -114,10 +114,10 @@ void launch(Mode mode, Args& a, unsigned char* words, bool compact, cudaStream_t
     const int guard = p.full && plain ? 0 : 2;
     const Shape shape{p.ctas(), p.threads, p.smem};
     switch (p.pz) {
-        case 1: launch_planes<1, true>(mode, kind, guard, shape, a, s); break;
-        case 2: launch_planes<2, true>(mode, kind, guard, shape, a, s); break;
-        case 3: launch_planes<3, true>(mode, kind, guard, shape, a, s); break;
-        default: launch_planes<4, true>(mode, kind, guard, shape, a, s); break;
+        case 1: return launch_planes<1, true>(mode, kind, guard, shape, a, query, s);
+        case 2: return launch_planes<2, true>(mode, kind, guard, shape, a, query, s);
+        case 3: return launch_planes<3, true>(mode, kind, guard, shape, a, query, s);
+        default: return launch_planes<4, true>(mode, kind, guard, shape, a, query, s);
     }
 }
 
@@ -132,25 +132,31 @@ size_t sor_grid_words(int n) {
     return bytes;
 }
 
+bool sor_grid_runs(const ProjectionArgs& p, SweepMode mode, bool compact) {
+    if (plan_for(p.g.n, compact).pz == 0) return false;
+    Args a = make_args(p, nullptr, nullptr, nullptr);
+    return launch(Mode(mode), a, nullptr, compact, true, nullptr);
+}
+
 void launch_sor_grid_fixed(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl, unsigned char* words,
                            bool compact, cudaStream_t s) {
     Args a = make_args(p, x, b, ctrl);
     a.subtract_mean = 1;
-    launch(kFixed, a, words, compact, s);
+    launch(kFixed, a, words, compact, false, s);
 }
 
 void launch_sor_grid_tolerance(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl,
                                unsigned char* words, bool compact, cudaStream_t s) {
     Args a = make_args(p, x, b, ctrl);
     a.subtract_mean = 1;
-    launch(kTolerance, a, words, compact, s);
+    launch(kTolerance, a, words, compact, false, s);
 }
 
 void launch_sor_grid_mixed(const ProjectionArgs& p, float* e, const float* r32, ProjControl* ctrl,
                            unsigned char* words, bool compact, cudaStream_t s) {
     Args a = make_args(p, e, r32, ctrl);
     a.flag_nonfinite = a.hw % 4 != 0;  // as the separate residual pass of those sizes does
-    launch(kMixed, a, words, compact, s);
+    launch(kMixed, a, words, compact, false, s);
 }
 
 }  // namespace vb

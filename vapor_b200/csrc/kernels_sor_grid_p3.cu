@@ -3,6 +3,6 @@
 
 namespace vb {
 namespace resident {
-template void launch_planes<3, true>(Mode, int, int, const Shape&, const Args&, cudaStream_t);
+template bool launch_planes<3, true>(Mode, int, int, const Shape&, const Args&, bool, cudaStream_t);
 }
 }  // namespace vb

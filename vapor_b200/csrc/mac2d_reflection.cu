@@ -529,7 +529,8 @@ public:
     ~Mac2DReflection() { cudaStreamSynchronize(st_.s); }
 
     const vapor_mac2d_refl_params& params() const { return p_; }
-    void set_wait_probe(int polls) { wait_probe_ = polls; }  // test hook
+    void set_wait_probe(int polls) { wait_probe_ = polls; }  // test hooks
+    void set_resident_sweeps(bool on) { resident_sweeps_ = on; }
     void set_params(const vapor_mac2d_refl_params& p) {
         p_ = p;
         patch_valid_ = false;
@@ -673,31 +674,40 @@ private:
     void sor(float dt, float h2, int iterations) {
         const int n = n_, G = ((n + 1) / 2 + 3) / 4;
         const int ctas = std::min(16, n / 2), rows = (n + ctas - 1) / ctas;
-        if (rows * G > 1024) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr;
+        const bool small = rows * G <= 512;
+        const auto kernel = small ? kr_sor_cluster<512> : kr_sor_cluster<1024>;
+        cfg.gridDim = dim3(unsigned(ctas));
+        cfg.blockDim = dim3(unsigned((rows * G + 31) / 32 * 32));
+        cfg.dynamicSmemBytes = size_t(2 * (rows + 2) * (4 * G + 4) + 32 * G) * sizeof(float);
+        cfg.stream = st_.s;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = unsigned(ctas);
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        if (cluster_fits_ < 0) {  // the device may have no cluster of that many SMs free
+            cluster_fits_ = 0;
+            if (rows * G <= 1024) {
+                static OncePerDevice once[2];
+                once[small]([&] {
+                    VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
+                    VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+                });
+                if (cudaOccupancyMaxActiveClusters(&cluster_fits_, kernel, &cfg) != cudaSuccess) {
+                    cudaGetLastError();
+                    cluster_fits_ = 0;
+                }
+            }
+        }
+        if (cluster_fits_ == 0 || !resident_sweeps_) {
             const long per_parity = long((n + 1) / 2) * n;
             for (int it = 0; it < iterations; ++it)
                 for (int parity = 0; parity < 2; ++parity)
                     kr_sor<<<blocks_r(per_parity), kT, 0, st_.s>>>(n, parity, p_.sor_omega, h2, dt, div_.p, pressure_.p);
             return;
         }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(unsigned(ctas));
-        cfg.blockDim = dim3(unsigned((rows * G + 31) / 32 * 32));
-        cfg.dynamicSmemBytes = size_t(2 * (rows + 2) * (4 * G + 4) + 32 * G) * sizeof(float);
-        cfg.stream = st_.s;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = unsigned(ctas);
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        static OncePerDevice once[2];
-        const bool small = rows * G <= 512;
-        const auto kernel = small ? kr_sor_cluster<512> : kr_sor_cluster<1024>;
-        once[small]([&] {
-            VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
-            VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        });
         VB_CUDA(cudaLaunchKernelEx(&cfg, kernel, n, iterations,
                                    p_.sor_omega, h2, dt, static_cast<const float*>(div_.p), pressure_.p, error_.p,
                                    wait_probe_));
@@ -745,6 +755,8 @@ private:
     int n_;
     vapor_mac2d_refl_params p_;
     int wait_probe_ = 0;
+    bool resident_sweeps_ = true;
+    int cluster_fits_ = -1;  // not known yet; else clusters of the sweeps that the device holds
     Stream st_;
     DevArray<float> smoke_, fwd_, back_, pressure_, div_, vx_, vy_, vxt_, vyt_, vxm_, vym_, vxh_, vyh_;
     DevArray<uint32_t> state_, special_;
@@ -837,6 +849,12 @@ VB_APIR vapor_status vapor_mac2d_refl_set_wait_probe(vapor_mac2d_refl* sim, int3
     return vb::guard([&] {
         require_r(sim && polls >= 0, "null handle or negative polls");
         sim->sim.set_wait_probe(polls);
+    });
+}
+VB_APIR vapor_status vapor_mac2d_refl_set_resident_sweeps(vapor_mac2d_refl* sim, int32_t enabled) {
+    return vb::guard([&] {
+        require_r(sim != nullptr, "null handle");
+        sim->sim.set_resident_sweeps(enabled != 0);
     });
 }
 VB_APIR vapor_status vapor_mac2d_refl_advance(vapor_mac2d_refl* sim, float dt) {

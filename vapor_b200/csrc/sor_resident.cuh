@@ -54,7 +54,7 @@ __host__ __device__ constexpr int max_threads(int pz) { return pz == 1 ? 768 : (
 
 // Weights and divisors: one for every cell, by diagonal, by a solid mask.
 enum Kind { kUniform = 0, kGeneral = 1, kMasked = 2 };
-enum Mode { kFixed = 0, kTolerance = 1, kMixed = 2 };
+enum Mode { kFixed = int(SweepMode::kFixed), kTolerance = int(SweepMode::kTolerance), kMixed = int(SweepMode::kMixed) };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -756,9 +756,10 @@ inline int row_floats(int hwp) {
 struct Shape {
     int ctas, threads, smem;
 };
-// Launches the kernel of this mode, kind and guard (sor_resident_launch.cuh).
+// Launches the kernel of this mode, kind and guard, or with `query` says whether
+// the device can hold the launch (sor_resident_launch.cuh).
 template <int PZ, bool GRID>
-void launch_planes(Mode mode, int kind, int guard, const Shape& p, const Args& a, cudaStream_t s);
+bool launch_planes(Mode mode, int kind, int guard, const Shape& p, const Args& a, bool query, cudaStream_t s);
 
 inline Args make_args(const ProjectionArgs& p, float* x, const float* b, ProjControl* ctrl) {
     Args a{};

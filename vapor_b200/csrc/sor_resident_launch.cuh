@@ -10,8 +10,35 @@
 namespace vb {
 namespace resident {
 
+// Whether the device can hold the launch: some devices have no cluster of that
+// many SMs free (a partition of the GPU, for one).
 template <int PZ, int MODE, int KIND, int GUARD, bool GRID>
-void launch_variant(const Shape& p, const Args& a, cudaStream_t s) {
+bool fits(const Shape& p, const cudaLaunchConfig_t& cfg) {
+    static std::mutex mutex;
+    static std::map<std::tuple<int, int, int, int>, bool> known;
+    int device = 0;
+    VB_CUDA(cudaGetDevice(&device));
+    const std::tuple<int, int, int, int> key(device, p.ctas, p.threads, p.smem);
+    std::lock_guard<std::mutex> lock(mutex);
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
+    const auto kernel = k_sor_resident<PZ, MODE, KIND, GUARD, GRID>;
+    int most = 0, sms = 0;
+    cudaError_t e;
+    if (GRID) {
+        VB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most, kernel, p.threads, size_t(p.smem));
+        most = most * sms >= p.ctas;
+    } else {
+        e = cudaOccupancyMaxActiveClusters(&most, kernel, &cfg);
+    }
+    if (e != cudaSuccess) cudaGetLastError();  // a shape that the device does not know
+    return known[key] = e == cudaSuccess && most > 0;
+}
+
+// Launches the kernel, or with `query` only says whether the device can hold it.
+template <int PZ, int MODE, int KIND, int GUARD, bool GRID>
+bool launch_variant(const Shape& p, const Args& a, bool query, cudaStream_t s) {
     const auto kernel = k_sor_resident<PZ, MODE, KIND, GUARD, GRID>;
     static OncePerDevice once;
     once([&] {
@@ -35,29 +62,31 @@ void launch_variant(const Shape& p, const Args& a, cudaStream_t s) {
     }
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
+    if (query) return fits<PZ, MODE, KIND, GUARD, GRID>(p, cfg);
     count_launch();
     VB_CUDA(cudaLaunchKernelEx(&cfg, kernel, a));
+    return true;
 }
 
 template <int PZ, int MODE, bool GRID>
-void launch_mode(int kind, int guard, const Shape& p, const Args& a, cudaStream_t s) {
+bool launch_mode(int kind, int guard, const Shape& p, const Args& a, bool query, cudaStream_t s) {
     if constexpr (MODE == kMixed)
-        if (kind == kMasked) return launch_variant<PZ, MODE, kMasked, 2, GRID>(p, a, s);
-    if (kind != kUniform) return launch_variant<PZ, MODE, kGeneral, 2, GRID>(p, a, s);
+        if (kind == kMasked) return launch_variant<PZ, MODE, kMasked, 2, GRID>(p, a, query, s);
+    if (kind != kUniform) return launch_variant<PZ, MODE, kGeneral, 2, GRID>(p, a, query, s);
     if constexpr (MODE != kTolerance) {
-        if (guard == 0) return launch_variant<PZ, MODE, kUniform, 0, GRID>(p, a, s);
+        if (guard == 0) return launch_variant<PZ, MODE, kUniform, 0, GRID>(p, a, query, s);
         if constexpr (!GRID)
-            if (guard == 1) return launch_variant<PZ, MODE, kUniform, 1, GRID>(p, a, s);
+            if (guard == 1) return launch_variant<PZ, MODE, kUniform, 1, GRID>(p, a, query, s);
     }
-    launch_variant<PZ, MODE, kUniform, 2, GRID>(p, a, s);
+    return launch_variant<PZ, MODE, kUniform, 2, GRID>(p, a, query, s);
 }
 
 template <int PZ, bool GRID>
-void launch_planes(Mode mode, int kind, int guard, const Shape& p, const Args& a, cudaStream_t s) {
+bool launch_planes(Mode mode, int kind, int guard, const Shape& p, const Args& a, bool query, cudaStream_t s) {
     switch (mode) {
-        case kFixed: launch_mode<PZ, kFixed, GRID>(kind, guard, p, a, s); break;
-        case kTolerance: launch_mode<PZ, kTolerance, GRID>(kind, guard, p, a, s); break;
-        default: launch_mode<PZ, kMixed, GRID>(kind, guard, p, a, s); break;
+        case kFixed: return launch_mode<PZ, kFixed, GRID>(kind, guard, p, a, query, s);
+        case kTolerance: return launch_mode<PZ, kTolerance, GRID>(kind, guard, p, a, query, s);
+        default: return launch_mode<PZ, kMixed, GRID>(kind, guard, p, a, query, s);
     }
 }
 

@@ -46,6 +46,7 @@ def _lib():
         f("vapor_mac2d_refl_set_params", _vp, R)
         f("vapor_mac2d_refl_advance", _vp, C.c_float)
         f("vapor_mac2d_refl_set_wait_probe", _vp, C.c_int32)
+        f("vapor_mac2d_refl_set_resident_sweeps", _vp, C.c_int32)
         f("vapor_mac2d_refl_reset", _vp)
         f("vapor_mac2d_refl_upload", _vp, _vp, _vp, _vp)
         f("vapor_mac2d_refl_download", _vp, _vp, _vp, _vp, _vp)
