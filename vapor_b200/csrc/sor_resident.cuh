@@ -129,6 +129,9 @@ __device__ __forceinline__ void send4(uint32_t addr, uint32_t second, const floa
 // false when the wait ran out.
 __device__ __forceinline__ bool receive4(uint32_t addr, uint32_t second, float* to, uint32_t epoch,
                                          int limit = kPollLimit) {
+    // unrolled, the polls' copies cost registers: a half sweep of a fixed budget
+    // 1.02 us at 45^3 and 1.61 at 49^3, with one copy 0.95 and 1.38
+#pragma unroll 1
     for (int i = 0; i < limit; ++i) {
         Words w;
         load_shared(addr, w.w[0], w.w[1]);
