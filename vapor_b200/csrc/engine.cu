@@ -311,8 +311,9 @@ void Workspace::set_solid(const uint8_t* mask) {
     if (fluid == 0) fail(VAPOR_INVALID_ARGUMENT, "the solid mask leaves no fluid cell");
     solid_.allocate(cells);
     solid_diag_.allocate(diag.size());
-    VB_CUDA(cudaMemcpy(solid_.p, nat.data(), cells, cudaMemcpyHostToDevice));
-    VB_CUDA(cudaMemcpy(solid_diag_.p, diag.data(), diag.size(), cudaMemcpyHostToDevice));
+    copy_in(solid_.p, nat.data(), cells, stream_);
+    copy_in(solid_diag_.p, diag.data(), diag.size(), stream_);
+    VB_CUDA(cudaStreamSynchronize(stream_));
     fluid_ = double(fluid);
 }
 

@@ -30,6 +30,14 @@ vapor_status guard(const std::function<void()>& f);
 void cuda_check(cudaError_t e, const char* what);
 #define VB_CUDA(call) ::vb::cuda_check((call), #call)
 
+// A host-to-device copy in the order of a stream. The library's streams do not
+// wait for the default stream, on which cudaMemcpy copies and returns while the
+// last part from pageable memory is still on its way. The caller synchronises the
+// stream before it gives the host memory back.
+inline void copy_in(void* to, const void* from, size_t bytes, cudaStream_t s) {
+    VB_CUDA(cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, s));
+}
+
 // Owning device allocation.
 template <class T>
 struct DevArray {

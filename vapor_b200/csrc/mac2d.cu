@@ -379,10 +379,10 @@ public:
     }
 
     void upload(const float* d, const float* u, const float* v) {
+        if (d) copy_in(d_.p, d, d_.bytes(), st_.s);
+        if (u) copy_in(u_.p, u, u_.bytes(), st_.s);
+        if (v) copy_in(v_.p, v, v_.bytes(), st_.s);
         VB_CUDA(cudaStreamSynchronize(st_.s));
-        if (d) VB_CUDA(cudaMemcpy(d_.p, d, d_.bytes(), cudaMemcpyHostToDevice));
-        if (u) VB_CUDA(cudaMemcpy(u_.p, u, u_.bytes(), cudaMemcpyHostToDevice));
-        if (v) VB_CUDA(cudaMemcpy(v_.p, v, v_.bytes(), cudaMemcpyHostToDevice));
     }
     void download(float* d, float* u, float* v) {
         VB_CUDA(cudaStreamSynchronize(st_.s));
@@ -495,8 +495,9 @@ private:
             if (patch_count_ > 0) {
                 patch_cells_.allocate(cells.size());
                 patch_weights_.allocate(weights.size());
-                VB_CUDA(cudaMemcpy(patch_cells_.p, cells.data(), cells.size() * 4, cudaMemcpyHostToDevice));
-                VB_CUDA(cudaMemcpy(patch_weights_.p, weights.data(), weights.size() * 4, cudaMemcpyHostToDevice));
+                copy_in(patch_cells_.p, cells.data(), cells.size() * 4, st_.s);
+                copy_in(patch_weights_.p, weights.data(), weights.size() * 4, st_.s);
+                VB_CUDA(cudaStreamSynchronize(st_.s));
             }
             patch_valid_ = true;
             patch_r_ = p.emitter_radius;

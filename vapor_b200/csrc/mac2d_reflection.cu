@@ -570,10 +570,10 @@ public:
     }
 
     void upload(const float* s, const float* u, const float* v) {
+        if (s) copy_in(smoke_.p, s, smoke_.bytes(), st_.s);
+        if (u) copy_in(vx_.p, u, vx_.bytes(), st_.s);
+        if (v) copy_in(vy_.p, v, vy_.bytes(), st_.s);
         VB_CUDA(cudaStreamSynchronize(st_.s));
-        if (s) VB_CUDA(cudaMemcpy(smoke_.p, s, smoke_.bytes(), cudaMemcpyHostToDevice));
-        if (u) VB_CUDA(cudaMemcpy(vx_.p, u, vx_.bytes(), cudaMemcpyHostToDevice));
-        if (v) VB_CUDA(cudaMemcpy(vy_.p, v, vy_.bytes(), cudaMemcpyHostToDevice));
     }
     void download(float* s, float* u, float* v, float* pr) {
         VB_CUDA(cudaStreamSynchronize(st_.s));
@@ -656,8 +656,9 @@ private:
             if (patch_count_ > 0) {
                 patch_cells_.allocate(2 * cells.size());
                 patch_weights_.allocate(weights.size());
-                VB_CUDA(cudaMemcpy(patch_cells_.p, cells.data(), cells.size() * sizeof(int2), cudaMemcpyHostToDevice));
-                VB_CUDA(cudaMemcpy(patch_weights_.p, weights.data(), weights.size() * 4, cudaMemcpyHostToDevice));
+                copy_in(patch_cells_.p, cells.data(), cells.size() * sizeof(int2), st_.s);
+                copy_in(patch_weights_.p, weights.data(), weights.size() * 4, st_.s);
+                VB_CUDA(cudaStreamSynchronize(st_.s));
             }
             patch_valid_ = true;
         }
