@@ -354,6 +354,7 @@ __global__ void __launch_bounds__(max_threads(PZ), 1) k_sor_resident(Args a) {
             if (from < 0) continue;
             const int second = tid + q * threads < 2 * per_block ? int(half_bytes) : y_half;
             Words w;
+#pragma unroll 1  // as in receive4
             for (int i = 0; !dead; ++i) {
                 const unsigned char* const at = a.words + from + c * 2 * second;
                 load_global(at, w.w[0], w.w[1]);
