@@ -499,11 +499,15 @@ void Workspace::project(const float* ui, const float* vi, const float* wi, float
     const bool graph = capturing_;
     const int interval = o.residual_check_interval;
     // Small and medium grids run their sweeps in one launch up to the next
-    // decision: in one cluster (16 SMs) where that is as fast, since several
-    // scenes then run side by side. Per half sweep, cluster against the whole
-    // device: 1.2 / 1.7 us at 48^3; at 50^3 fixed budgets 2.1 / 1.6 and tolerance
-    // checks 2.7 / 2.1, the mixed solver 1.8 / 1.9; at 64^3 1.9 / 1.4, 2.9 / 1.9
-    // and 1.8 / 1.6.
+    // decision: in one cluster (16 SMs), since several scenes then run side by
+    // side, or on the whole device. Per half sweep, cluster against the whole
+    // device, in us: fixed budgets 1.48 / 1.32 at 50^3, 1.44 / 1.32 at 56^3, 1.60
+    // / 1.20 at 60^3, 1.55 / 1.11 at 64^3; with tolerance checks 2.11 / 1.81, 2.28
+    // / 1.81, 2.47 / 1.68, 2.46 / 1.57; the mixed solver 1.38 / 1.64, 1.41 / 1.67,
+    // 1.54 / 1.50, 1.51 / 1.38 (a plume step to 1e-6: 2.23 / 2.58, 2.69 / 3.09,
+    // 3.21 / 3.10, 3.41 / 3.12 ms). So the mixed solver stays in the cluster as far
+    // as that reaches; from 60^3 on a scene alone would gain 3 to 8% of its step
+    // from the whole device.
     // Where the device cannot hold the one, the other runs, or launches per colour.
     const bool resident = resident_sweeps_ && !fpcg && sor_block_iterations(n_) == 0;
     const bool grid_first = !sor_cluster_applies(n_) || (!mixed && !shared_device_);

@@ -17,10 +17,10 @@
 // reader polls. So a half sweep costs one block barrier and one store to a
 // neighbour SM, with no fence and no barrier over the cluster (st.async with
 // complete_tx bytes, or stores with an arrival per warp on a remote mbarrier,
-// took 0.4 us more a half sweep). Measured per half sweep: 0.41 us at 16^3,
-// 0.48 at 32^3 and 0.83 at 48^3, bound by that chain of shared-memory loads,
-// seven dependent additions, barrier and neighbour store; 1.6 at 64^3, bound
-// by the issue slots of 16 SMs. Hence the shape of the update: what a slot's
+// took 0.4 us more a half sweep). Measured per half sweep of a fixed
+// budget: 0.40 us at 16^3, 0.46 at 32^3 and 0.83 at 48^3, bound by that chain of
+// shared-memory loads, seven dependent additions, barrier and neighbour store;
+// 1.55 at 64^3 (mixed 1.51), bound by the issue slots of 16 SMs. Hence the shape of the update: what a slot's
 // place selects is constant per warp (rows of one parity share a warp) or per
 // launch (GUARD, KIND), and parameters are not indexed by the diagonal (an
 // indexed parameter read replays per diagonal met in the warp).

@@ -2,10 +2,13 @@
 // one pass over a large grid: the mixed solver's sweeps and the FPCG
 // preconditioner's smoothing on unmasked grids with n % 8 == 0.
 //
-// One launch per colour moves 24 bytes a cell for an iteration; at 256^3, where
-// iterate and right-hand side (134 MB) do not stay in L2, DRAM bounds it at 46 us
-// an iteration (cache hints and a serpentine order of the planes changed that by
-// less than 5%). This pass reads both once for two iterations.
+// One launch per colour reads iterate and right-hand side anew for every colour:
+// at 256^3, where they (134 MB) do not stay in L2, the two launches of an
+// iteration move 224 MB, 13.4 bytes a cell, in 46 us. The latency of the
+// neighbour rows' loads bounds them, at 59% of the DRAM throughput and 64% of the
+// issue slots (cache hints and a serpentine order of the planes changed the time
+// by less than 5%). This pass reads both once for two iterations: 199 MB, 6 bytes
+// a cell and iteration.
 //
 // A CTA owns a tile of 64 cells in x by up to 56 rows in y and a chunk of planes,
 // and marches up the chunk: at step tau plane tau arrives, half sweep t = 1 .. 4
